@@ -68,6 +68,7 @@ struct nb_handle {
     int jsplit = 1;
     int tj = 256;               // sources per packed j-tile (128, 256, 512)
     int stages = 4;             // depth of the force kernel's copy ring
+    double* fp64_partial = nullptr;  // split FP64 sums (arena, FP64 handles only)
     int jalloc = 1;             // j-split the arena's partial buffer holds
     float* jpartial = nullptr;  // j-split partials (arena)
     int64_t jstride = 0;
@@ -269,7 +270,7 @@ cudaError_t enqueue_force(nb_handle* h, const nb::Targets& tg, cudaStream_t s, b
             t2.d_count = &h->clk->n_active;
         }
         nb::Sources64 src{h->x, h->y, h->z, h->m, h->n};
-        return nb::launch_force_fp64(h->p.law, pot, src, t2, h->p.G, &h->clk->err, s);
+        return nb::launch_force_fp64(h->p.law, pot, src, t2, h->p.G, h->fp64_partial, s);
     }
     // Morton order of the sources keeps every j-tile compact, so the FP32
     // coordinates relative to its origin stay small.
@@ -471,7 +472,8 @@ cudaError_t capture_output_graph(nb_handle* h, cudaGraphExec_t* out, bool sort) 
 
 int ensure_capacity(nb_handle* h, int64_t n) {
     const int js_need = h->auto_cfg ? kAutoJsplitMax : h->jsplit;
-    if (n <= h->cap && h->arena && js_need <= h->jalloc) return NB_OK;
+    const bool fp64 = h->p.precision == NB_PREC_FP64;
+    if (n <= h->cap && h->arena && js_need <= h->jalloc && (!fp64 || h->fp64_partial)) return NB_OK;
     drop_graph(h);
     if (h->arena) {
         cudaFree(h->arena);
@@ -507,6 +509,7 @@ int ensure_capacity(nb_handle* h, int64_t n) {
     size_t o_ext = take(sizeof(float4) * (size_t)ntiles);
     size_t o_ds = take(sizeof(double) * (size_t)dblocks);
     size_t o_do = take(sizeof(double) * 8);
+    size_t o_fp = take(fp64 ? nb::fp64_partial_bytes() : 0);
     void* a = nullptr;
     NB_CK(cudaMalloc(&a, off));
     char* b = static_cast<char*>(a);
@@ -539,6 +542,7 @@ int ensure_capacity(nb_handle* h, int64_t n) {
     h->diag_scratch = (double*)(b + o_ds);
     h->diag_blocks = dblocks / 8;
     h->diag_out = (double*)(b + o_do);
+    h->fp64_partial = fp64 ? (double*)(b + o_fp) : nullptr;
     h->ntiles = (int32_t)((n + h->tj - 1) / h->tj);
     return NB_OK;
 }

@@ -9,11 +9,36 @@
 //
 // Sources are staged through shared memory in tiles of kTile (x, y, z, m);
 // one target per thread.
+//
+// What bounds it: the FP64 pipe (2 lanes per clock and SM on this GPU), about
+// 60 FP64-pipe operations per pair, so the time is pairs / (busy SMs).  One
+// block of targets per CTA leaves most SMs idle below 152 x 8 blocks (N =
+// 4096: 32 CTAs on 152 SMs, 8.0 ms a force), so each block's sources are
+// split over js CTAs (fp64_split) whose compensated partial sums are joined
+// in part order by k_force_fp64_join: 1.76 ms a step at N = 4096, the rate
+// of a full GPU (9.6 G interactions/s).
 #include "nb_internal.cuh"
 
 namespace nb {
 
 constexpr int kTile = 128;
+constexpr int kFp64Items = 8 * 152;   // (block, part) items a split evaluation aims at
+constexpr int64_t kFp64MinPart = 32;  // fewest sources in a part
+
+// Parts that each block of targets is split into.  Up to kFp64Items items in
+// all: 8 CTAs of 128 threads fill an SM (60 registers), the items of one wave
+// differ by at most 1 in 8 between SMs, and the partials stay within a fixed
+// scratch (fp64_partial_bytes).  From kFp64Items / 2 blocks of targets on
+// there is nothing to split.  Depends on the counts only, so the sums do not
+// depend on scheduling; with an active list the count is the device's.
+__host__ __device__ __forceinline__ int fp64_split(int64_t nblocks, int64_t nsrc) {
+    int64_t js = nblocks > 0 ? kFp64Items / nblocks : 1;
+    const int64_t most = nsrc / kFp64MinPart;
+    if (js > most) js = most;
+    return js < 1 ? 1 : (int)js;
+}
+
+size_t fp64_partial_bytes() { return sizeof(double) * 8 * (size_t)kFp64Items * kTile; }
 
 template <int LAW>
 __device__ __forceinline__ void pair_force64(double px, double py, double pz, dvec4 q, double G,
@@ -70,12 +95,16 @@ __device__ __forceinline__ double pair_pot64(double px, double py, double pz, dv
 }
 
 template <int LAW, bool ACC, bool POT>
-__global__ void __launch_bounds__(kTile) k_force_fp64(Sources64 src, Targets tg, double G) {
+__global__ void __launch_bounds__(kTile)
+    k_force_fp64(Sources64 src, Targets tg, double G, double* __restrict__ partial) {
     __shared__ dvec4 sj[kTile];
     const int64_t ntg = tg.d_count ? (int64_t)(*tg.d_count) : tg.n;
-    const int64_t base = (int64_t)blockIdx.x * kTile;
-    if (base >= ntg) return;
-    const int64_t t = base + threadIdx.x;
+    const int64_t nblocks = (ntg + kTile - 1) / kTile;
+    const int js = fp64_split(nblocks, src.n);
+    const int64_t blk = (int64_t)blockIdx.x / js;
+    const int part = (int)((int64_t)blockIdx.x % js);
+    if (blk >= nblocks) return;  // CTA-uniform
+    const int64_t t = blk * kTile + threadIdx.x;
     int32_t p = -1;
     double px = 0.0, py = 0.0, pz = 0.0, h = tg.h_const;
     if (t < ntg) {
@@ -89,12 +118,13 @@ __global__ void __launch_bounds__(kTile) k_force_fp64(Sources64 src, Targets tg,
     const double h3_inv = h_inv * h_inv * h_inv;
     double sx = 0.0, sy = 0.0, sz = 0.0, sp = 0.0;
     double cx = 0.0, cy = 0.0, cz = 0.0, cp = 0.0;
-    for (int64_t j0 = 0; j0 < src.n; j0 += kTile) {
+    const int64_t jlo = src.n * part / js, jhi = src.n * (part + 1) / js;
+    for (int64_t j0 = jlo; j0 < jhi; j0 += kTile) {
         __syncthreads();
         const int64_t jj = j0 + threadIdx.x;
-        if (jj < src.n) sj[threadIdx.x] = make_dvec4(src.x[jj], src.y[jj], src.z[jj], src.m[jj]);
+        if (jj < jhi) sj[threadIdx.x] = make_dvec4(src.x[jj], src.y[jj], src.z[jj], src.m[jj]);
         __syncthreads();
-        const int cnt = (int)((src.n - j0) < kTile ? (src.n - j0) : kTile);
+        const int cnt = (int)((jhi - j0) < kTile ? (jhi - j0) : kTile);
         for (int j = 0; j < cnt; ++j) {
             const dvec4 q = sj[j];
             if (ACC) {
@@ -107,6 +137,23 @@ __global__ void __launch_bounds__(kTile) k_force_fp64(Sources64 src, Targets tg,
             if (POT) two_sum_acc(sp, cp, pair_pot64<LAW>(px, py, pz, q, G, h, h_inv));
         }
     }
+    if (js > 1) {
+        // compensated sums of this part, one row of kTile per quantity
+        double* q = partial + (blk * js + part) * (8 * kTile) + threadIdx.x;
+        if (ACC) {
+            q[0 * kTile] = sx;
+            q[1 * kTile] = cx;
+            q[2 * kTile] = sy;
+            q[3 * kTile] = cy;
+            q[4 * kTile] = sz;
+            q[5 * kTile] = cz;
+        }
+        if (POT) {
+            q[6 * kTile] = sp;
+            q[7 * kTile] = cp;
+        }
+        return;
+    }
     if (p < 0) return;
     if (ACC) {
         tg.ax[p] = sx + cx;
@@ -116,25 +163,69 @@ __global__ void __launch_bounds__(kTile) k_force_fp64(Sources64 src, Targets tg,
     if (POT) tg.pot[p] = sp + cp;
 }
 
+// Adds the parts of every target in part order, sums with TwoSum and carries
+// beside them, so a split evaluation keeps the accuracy of an unsplit one.
+template <bool ACC, bool POT>
+__global__ void __launch_bounds__(kTile)
+    k_force_fp64_join(int64_t nsrc, Targets tg, const double* __restrict__ partial) {
+    const int64_t ntg = tg.d_count ? (int64_t)(*tg.d_count) : tg.n;
+    const int64_t nblocks = (ntg + kTile - 1) / kTile;
+    const int js = fp64_split(nblocks, nsrc);
+    const int64_t t = (int64_t)blockIdx.x * kTile + threadIdx.x;
+    if (js == 1 || t >= ntg) return;
+    const int32_t p = tg.idx ? tg.idx[t] : (int32_t)t;
+    double s[4] = {0.0, 0.0, 0.0, 0.0}, c[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int part = 0; part < js; ++part) {
+        const double* q = partial + ((int64_t)blockIdx.x * js + part) * (8 * kTile) + threadIdx.x;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (k < 3 ? !ACC : !POT) continue;
+            two_sum_acc(s[k], c[k], q[(2 * k) * kTile]);
+            c[k] += q[(2 * k + 1) * kTile];
+        }
+    }
+    if (ACC) {
+        tg.ax[p] = s[0] + c[0];
+        tg.ay[p] = s[1] + c[1];
+        tg.az[p] = s[2] + c[2];
+    }
+    if (POT) tg.pot[p] = s[3] + c[3];
+}
+
 template <int LAW>
 static cudaError_t launch_law(bool acc, bool pot, const Sources64& src, const Targets& tg,
-                              double G, cudaStream_t s) {
-    const int64_t grid = (tg.n + kTile - 1) / kTile;
-    if (grid <= 0) return cudaSuccess;
+                              double G, double* partial, cudaStream_t s) {
+    const int64_t nblocks = (tg.n + kTile - 1) / kTile;
+    if (nblocks <= 0) return cudaSuccess;
+    // an active list may leave any number of blocks up to nblocks, split further the fewer they are
+    const int js = fp64_split(nblocks, src.n);
+    const bool split = js > 1 || (tg.d_count && fp64_split(1, src.n) > 1);
+    int64_t grid = nblocks * js;
+    if (tg.d_count && split && grid < kFp64Items) grid = kFp64Items;
     if (acc && pot)
-        k_force_fp64<LAW, true, true><<<(unsigned)grid, kTile, 0, s>>>(src, tg, G);
+        k_force_fp64<LAW, true, true><<<(unsigned)grid, kTile, 0, s>>>(src, tg, G, partial);
     else if (acc)
-        k_force_fp64<LAW, true, false><<<(unsigned)grid, kTile, 0, s>>>(src, tg, G);
+        k_force_fp64<LAW, true, false><<<(unsigned)grid, kTile, 0, s>>>(src, tg, G, partial);
     else if (pot)
-        k_force_fp64<LAW, false, true><<<(unsigned)grid, kTile, 0, s>>>(src, tg, G);
+        k_force_fp64<LAW, false, true><<<(unsigned)grid, kTile, 0, s>>>(src, tg, G, partial);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess || !split) return e;
+    // blocks that can be split: at most kFp64Items / 2
+    const int64_t jb = nblocks < kFp64Items / 2 ? nblocks : kFp64Items / 2;
+    if (acc && pot)
+        k_force_fp64_join<true, true><<<(unsigned)jb, kTile, 0, s>>>(src.n, tg, partial);
+    else if (acc)
+        k_force_fp64_join<true, false><<<(unsigned)jb, kTile, 0, s>>>(src.n, tg, partial);
+    else if (pot)
+        k_force_fp64_join<false, true><<<(unsigned)jb, kTile, 0, s>>>(src.n, tg, partial);
     return cudaGetLastError();
 }
 
 cudaError_t launch_force_fp64(int law, bool pot, const Sources64& src, const Targets& tg,
-                              double G, uint32_t* /*err*/, cudaStream_t s) {
+                              double G, double* partial, cudaStream_t s) {
     const bool acc = tg.ax != nullptr;
-    if (law == NB_LAW_PLUMMER) return launch_law<NB_LAW_PLUMMER>(acc, pot, src, tg, G, s);
-    return launch_law<NB_LAW_SPLINE_G2>(acc, pot, src, tg, G, s);
+    if (law == NB_LAW_PLUMMER) return launch_law<NB_LAW_PLUMMER>(acc, pot, src, tg, G, partial, s);
+    return launch_law<NB_LAW_SPLINE_G2>(acc, pot, src, tg, G, partial, s);
 }
 
 }  // namespace nb

@@ -298,8 +298,11 @@ cudaError_t launch_force_mixed(int law, bool pot, const Sources32& src, const Ta
                                double G, uint32_t* err, int block, int ipt, cudaStream_t s,
                                int stages = 4);
 bool tile_size_ok(int tile_j);
+// partial: scratch of fp64_partial_bytes() for evaluations whose sources are
+// split over several CTAs (few targets).
 cudaError_t launch_force_fp64(int law, bool pot, const Sources64& src, const Targets& tg,
-                              double G, uint32_t* err, cudaStream_t s);
+                              double G, double* partial, cudaStream_t s);
+size_t fp64_partial_bytes();
 
 // Integrator kernels (nb_integrate.cu).
 // Active list (Ti_endstep == t_int); slots are scanned in perm order when perm
