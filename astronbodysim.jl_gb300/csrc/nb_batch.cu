@@ -8,9 +8,9 @@
 //   admission and every 64 of their own steps; large ones by a radix sort of
 //   their own particles every step) -> per-system packed FP32 tiles -> force
 //   over whole i-blocks with the kick in its epilogue -> step counter.
-// The force kernel never splits an i-block and a system's order depends only
-// on its own particles, so a system's trajectory is bit-identical whether it
-// runs alone or among others.
+// A system's order and the split of its work depend only on its own particles
+// and their number, so its trajectory is bit-identical whether it runs alone or
+// among others.
 #include <algorithm>
 
 #include "nb_pairs.cuh"
@@ -412,10 +412,19 @@ __global__ void __launch_bounds__(kTileJ)
 }
 
 // ---------------------------------------------------------------------------
-// Force over whole i-blocks.  items[k] = (rank, i-block), largest systems
-// first; persistent CTAs claim items from a device counter.  Within an item
-// the CTA streams all j-tiles of that system through the bulk-copy ring, in
-// order, exactly like the single-system kernel.
+// Force over i-blocks.  items[k] = (rank, i-block, part of the j-tiles),
+// largest systems first; persistent CTAs claim items from a device counter.
+// Within an item the CTA streams the j-tiles of its part through the bulk-copy
+// ring, in order, exactly like the single-system kernel.
+//
+// Why the j-tiles of the larger systems are split: one item over all tiles of
+// a system takes ntiles x 17 us (256 x 256 pairs at a CTA's share of the GPU),
+// 3 ms at N = 45 000, and a step cannot end before its longest item: a mix of
+// 12 systems of 413 .. 45 387 particles spent 3.24 ms a step on work that
+// fills the GPU for 0.8 ms.  A part's sums go to global memory as compensated
+// pairs; the part that finishes last (a counter per split block) adds them in
+// part order, so the result does not depend on which CTA that is.  Integrating
+// that mix for 5 .. 15 steps took 56.5 ms unsplit and takes 21.8 ms.
 // ---------------------------------------------------------------------------
 // Launch shapes (threads per CTA, targets per thread); an item is one i-block
 // of BLOCK * IPT targets.  Default 128 x 2; the engine takes the shape from its
@@ -456,6 +465,24 @@ __device__ __forceinline__ void kick_particle(double* __restrict__ vx, double* _
     }
 }
 
+// Parts of a system's j-tiles: at least kPartTiles tiles each (the join then
+// costs below 1 % of a part), at most kMaxParts, and no more than it takes to
+// have kPartItems items, from where on the blocks alone balance the GPU.  A
+// rule on the system's own size, so a system is split the same way alone and
+// in any mix.
+constexpr int kPartTiles = 8, kMaxParts = 8, kPartItems = 4096;
+
+int batch_parts(int64_t n, int block, int ipt) {
+    const int64_t nt = (n + kTileJ - 1) / kTileJ, bt = (int64_t)block * ipt, nb = (n + bt - 1) / bt;
+    if (nb < 1) return 1;
+    const int64_t p = std::min<int64_t>({nt / kPartTiles, kMaxParts, kPartItems / nb});
+    return p < 1 ? 1 : (int)p;
+}
+
+int batch_max_parts() { return kMaxParts; }
+
+size_t batch_partial_row(int block, int ipt) { return (size_t)8 * block * ipt; }
+
 template <int LAW, bool ACC, bool POT, int BLOCK, int IPT>
 __global__ void __launch_bounds__(BLOCK, (BatchOcc<BLOCK, IPT, ACC, POT>::value))
     k_force_batch(BatchForce f) {
@@ -464,7 +491,7 @@ __global__ void __launch_bounds__(BLOCK, (BatchOcc<BLOCK, IPT, ACC, POT>::value)
     __shared__ __align__(128) float4 buf[kStages * kTileJ];
     __shared__ __align__(8) uint64_t full[kStages];
     __shared__ uint32_t done[kStages];
-    __shared__ int32_t item_sh;
+    __shared__ int32_t item_sh, last_sh;
     __shared__ uint32_t abort_sh;
     __shared__ float2 tpx[kFBt], tpy[kFBt], tpz[kFBt];
     const int tid = threadIdx.x, lane = tid & 31;
@@ -487,8 +514,8 @@ __global__ void __launch_bounds__(BLOCK, (BatchOcc<BLOCK, IPT, ACC, POT>::value)
         __syncthreads();
         const int32_t it = item_sh;
         if (it >= f.nitems || abort_sh) break;  // CTA-uniform
-        const int2 ib = f.items[it];
-        const SysDesc& d = f.sys[ib.x];
+        const BatchItem ib = f.items[it];
+        const SysDesc& d = f.sys[ib.rank];
         if (f.nsteps_slot) {
             // a system that has made all its steps keeps its state: no force,
             // no kick (CTA-uniform: every thread reads the same words)
@@ -498,12 +525,15 @@ __global__ void __launch_bounds__(BLOCK, (BatchOcc<BLOCK, IPT, ACC, POT>::value)
                 continue;
             }
         }
-        const int32_t ntiles = d.ntiles;
+        // tiles t_lo .. t_lo + ntiles of this part
+        const int32_t t_lo = (int32_t)((int64_t)ib.part * d.ntiles / ib.nparts);
+        const int32_t ntiles = (int32_t)((int64_t)(ib.part + 1) * d.ntiles / ib.nparts) - t_lo;
+        const int32_t tile0 = d.tile_off + t_lo;
         if (tid == 0) {
             for (int k = 0; k < kStages && k < ntiles; ++k) {
                 const uint32_t v = vbase + k;
                 mbar_arrive_expect_tx(&full[v % kStages], kTileJ * sizeof(float4));
-                bulk_g2s(&buf[(v % kStages) * kTileJ], f.pack + (int64_t)(d.tile_off + k) * kTileJ,
+                bulk_g2s(&buf[(v % kStages) * kTileJ], f.pack + (int64_t)(tile0 + k) * kTileJ,
                          kTileJ * sizeof(float4), &full[v % kStages]);
                 last_issued = v + 1;
             }
@@ -512,7 +542,7 @@ __global__ void __launch_bounds__(BLOCK, (BatchOcc<BLOCK, IPT, ACC, POT>::value)
         float hh[IPT], h2[IPT];
 #pragma unroll
         for (int k = 0; k < IPT; ++k) {
-            const int32_t slot = ib.y * kFBt + k * BLOCK + tid;
+            const int32_t slot = ib.block * kFBt + k * BLOCK + tid;
             pidx[k] = -1;
             double x = 0.0, y = 0.0, z = 0.0;
             if (slot < d.n) {
@@ -540,7 +570,7 @@ __global__ void __launch_bounds__(BLOCK, (BatchOcc<BLOCK, IPT, ACC, POT>::value)
             const uint32_t v = vbase + t;
             const int st = (int)(v % kStages);
             const uint32_t par = (v / kStages) & 1u;
-            const float4 oh = f.origin[d.tile_off + t].hi, ol = f.origin[d.tile_off + t].lo;
+            const float4 oh = f.origin[tile0 + t].hi, ol = f.origin[tile0 + t].lo;
             float xr[IPT], yr[IPT], zr[IPT];
 #pragma unroll
             for (int k = 0; k < IPT; ++k) {
@@ -560,11 +590,11 @@ __global__ void __launch_bounds__(BLOCK, (BatchOcc<BLOCK, IPT, ACC, POT>::value)
                 break;
             }
             const float4* b = &buf[st * kTileJ];
-            const float4 ex = f.ext[d.tile_off + t];
+            const float4 ex = f.ext[tile0 + t];
             bool near = false;
             if (LAW == NB_LAW_SPLINE_G2) near = warp_near<IPT>(ex, xr, yr, zr, hh, pidx);
             // the system's last tile may be partial
-            const int np2 = tile_pairs<kTileJ>(d.n - t * kTileJ);
+            const int np2 = tile_pairs<kTileJ>(d.n - (t_lo + t) * kTileJ);
             if (near)
                 pair_loop_checked<LAW, ACC, POT, IPT>(b, xr, yr, zr, hh, h2, ax, ay, az, ap, ex.w, np2);
             else if (ex.w > 0.0f && warp_expandable<IPT>(ex, oh.w, xr, yr, zr, pidx))
@@ -581,7 +611,7 @@ __global__ void __launch_bounds__(BLOCK, (BatchOcc<BLOCK, IPT, ACC, POT>::value)
                     if (t + kStages < ntiles) {
                         mbar_arrive_expect_tx(&full[st], kTileJ * sizeof(float4));
                         bulk_g2s(&buf[st * kTileJ],
-                                 f.pack + (int64_t)(d.tile_off + t + kStages) * kTileJ,
+                                 f.pack + (int64_t)(tile0 + t + kStages) * kTileJ,
                                  kTileJ * sizeof(float4), &full[st]);
                     }
                 }
@@ -596,7 +626,57 @@ __global__ void __launch_bounds__(BLOCK, (BatchOcc<BLOCK, IPT, ACC, POT>::value)
                 if (POT) two_sum_acc(sp[k], cp[k], ap[k]);
             }
         }
-        if (!timed_out) {
+        bool write = !timed_out;
+        if (ib.nparts > 1) {
+            // this part's compensated sums, one row of kFBt per quantity
+            constexpr size_t kRow = (size_t)8 * kFBt;
+            float* q0 = f.partial + (size_t)ib.prow * kRow + tid;
+            if (!timed_out) {
+                float* q = q0 + ib.part * kRow;
+#pragma unroll
+                for (int k = 0; k < IPT; ++k) {
+                    const float v[8] = {sx[k], cx[k], sy[k], cy[k], sz[k], cz[k], sp[k], cp[k]};
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (j < 6 ? ACC : POT) __stcg(q + j * kFBt + k * BLOCK, v[j]);
+                }
+            }
+            __threadfence();  // the sums before the count
+            __syncthreads();
+            // a part that gave up is not counted: its block is then not joined
+            if (tid == 0)
+                last_sh = abort_sh ? 0 : atomicAdd(f.counter + 1 + ib.done, 1) == ib.nparts - 1;
+            __syncthreads();
+            write = write && last_sh;
+            if (write) {
+                __threadfence();  // the count before the other parts' sums
+#pragma unroll
+                for (int k = 0; k < IPT; ++k) {
+                    sx[k] = sy[k] = sz[k] = sp[k] = 0.0f;
+                    cx[k] = cy[k] = cz[k] = cp[k] = 0.0f;
+                }
+                for (int part = 0; part < ib.nparts; ++part) {
+                    const float* q = q0 + part * kRow;
+#pragma unroll
+                    for (int k = 0; k < IPT; ++k) {
+                        const float* r = q + k * BLOCK;
+                        if (ACC) {
+                            two_sum_acc(sx[k], cx[k], __ldcg(r));
+                            cx[k] += __ldcg(r + kFBt);
+                            two_sum_acc(sy[k], cy[k], __ldcg(r + 2 * kFBt));
+                            cy[k] += __ldcg(r + 3 * kFBt);
+                            two_sum_acc(sz[k], cz[k], __ldcg(r + 4 * kFBt));
+                            cz[k] += __ldcg(r + 5 * kFBt);
+                        }
+                        if (POT) {
+                            two_sum_acc(sp[k], cp[k], __ldcg(r + 6 * kFBt));
+                            cp[k] += __ldcg(r + 7 * kFBt);
+                        }
+                    }
+                }
+            }
+        }
+        if (write) {
 #pragma unroll
             for (int k = 0; k < IPT; ++k) {
                 const int32_t p = pidx[k];
@@ -646,7 +726,7 @@ static int occ_of() {
 
 template <int LAW, bool ACC, bool POT, int B, int I>
 static cudaError_t launch_of(const BatchForce& f, int grid, cudaStream_t s) {
-    cudaError_t e = cudaMemsetAsync(f.counter, 0, sizeof(int32_t), s);
+    cudaError_t e = cudaMemsetAsync(f.counter, 0, sizeof(int32_t) * (1 + (size_t)f.nsplit), s);
     if (e != cudaSuccess) return e;
     k_force_batch<LAW, ACC, POT, B, I><<<grid, B, 0, s>>>(f);
     return cudaGetLastError();

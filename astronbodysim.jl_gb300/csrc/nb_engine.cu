@@ -90,9 +90,14 @@ struct nb_engine {
     double* dt_slot = nullptr;
     double* fac_step = nullptr;
     double* fac_once = nullptr;
-    int2* items = nullptr;
-    int2* items_new = nullptr;
+    nb::BatchItem* items = nullptr;
+    nb::BatchItem* items_new = nullptr;
     int32_t* counter = nullptr;
+    // partial sums of the systems whose j-tiles are split: grown in rebuild()
+    // to what the running systems need, freed with the engine
+    float* partial = nullptr;
+    size_t partial_floats = 0;
+    bool split = true;  // false: no memory for the partial sums, whole i-blocks instead
     uint32_t* derr = nullptr;
     int64_t tile_cap = 0;
     int64_t item_cap = 0;
@@ -108,6 +113,7 @@ struct nb_engine {
     int32_t nrank = 0;
     int32_t ntiles_total = 0;
     int32_t nitems = 0;
+    int32_t nsplit = 0;  // split blocks among them
     int32_t max_small_n = 0;   // largest system ordered in shared memory
     // systems too large for the shared-memory sort ("large"): their ranks,
     // particle count and largest size; they are radix-sorted every step
@@ -203,6 +209,22 @@ int check_err(nb_engine* e) {
     return NB_OK;
 }
 
+// Appends the work items of the system of rank r: its i-blocks, each in
+// batch_parts() parts.  prow and nsplit count the rows of partial sums and the
+// split blocks so far.
+void add_items(nb_engine* e, std::vector<nb::BatchItem>& items, int32_t r, const nb::SysDesc& d,
+               int64_t& prow, int32_t& nsplit) {
+    const int32_t parts = e->split ? nb::batch_parts(d.n, e->fblock, e->fipt) : 1;
+    for (int32_t b = 0; b < d.nblocks; ++b) {
+        for (int32_t k = 0; k < parts; ++k)
+            items.push_back(nb::BatchItem{r, b, k, parts, (int32_t)prow, nsplit});
+        if (parts > 1) {
+            prow += parts;
+            nsplit += 1;
+        }
+    }
+}
+
 // Rebuild the rank tables of the running systems and upload them.
 int rebuild(nb_engine* e) {
     std::vector<int32_t> slots;
@@ -253,16 +275,38 @@ int rebuild(nb_engine* e) {
     for (int32_t r = 0; r < R; ++r) order[r] = r;
     std::stable_sort(order.begin(), order.end(),
                      [&](int32_t a, int32_t b) { return sd[a].ntiles > sd[b].ntiles; });
-    std::vector<int2> items;
-    for (int32_t r : order)
-        for (int32_t b = 0; b < sd[r].nblocks; ++b) items.push_back(make_int2(r, b));
+    std::vector<nb::BatchItem> items;
+    int64_t prow = 0;
+    int32_t nsplit = 0;
+    e->split = true;
+    for (int32_t r : order) add_items(e, items, r, sd[r], prow, nsplit);
+    const size_t pf = (size_t)prow * nb::batch_partial_row(e->fblock, e->fipt);
+    if (pf > e->partial_floats) {
+        if (e->partial) cudaFree(e->partial);
+        e->partial = nullptr;
+        e->partial_floats = 0;
+        const cudaError_t me = cudaMalloc(&e->partial, sizeof(float) * pf);
+        if (me == cudaSuccess) {
+            e->partial_floats = pf;
+        } else if (me == cudaErrorMemoryAllocation) {
+            (void)cudaGetLastError();
+            e->partial = nullptr;
+            e->split = false;
+            items.clear();
+            prow = 0;
+            nsplit = 0;
+            for (int32_t r : order) add_items(e, items, r, sd[r], prow, nsplit);
+        } else {
+            NE_CK(me);
+        }
+    }
     if (toff > e->tile_cap) return efail(e, NB_ERR_STATE, "tile capacity exceeded");
     if ((int64_t)items.size() > e->item_cap) return efail(e, NB_ERR_STATE, "work-item capacity exceeded");
     if (R > 0) {
         NE_CK(cudaMemcpy(e->sysdesc, sd.data(), sizeof(nb::SysDesc) * R, cudaMemcpyHostToDevice));
         NE_CK(cudaMemcpy(e->batchsys, bs.data(), sizeof(nb::BatchSys) * R, cudaMemcpyHostToDevice));
         NE_CK(cudaMemcpy(e->tile_rank, trank.data(), sizeof(int32_t) * toff, cudaMemcpyHostToDevice));
-        NE_CK(cudaMemcpy(e->items, items.data(), sizeof(int2) * items.size(), cudaMemcpyHostToDevice));
+        NE_CK(cudaMemcpy(e->items, items.data(), sizeof(nb::BatchItem) * items.size(), cudaMemcpyHostToDevice));
     }
     NE_CK(cudaMemcpy(e->rank_of_slot, ros.data(), sizeof(int32_t) * ros.size(), cudaMemcpyHostToDevice));
     NE_CK(cudaMemcpy(e->fac_step, fstep.data(), sizeof(double) * fstep.size(), cudaMemcpyHostToDevice));
@@ -271,6 +315,7 @@ int rebuild(nb_engine* e) {
     e->nrank = R;
     e->ntiles_total = (int32_t)toff;
     e->nitems = (int32_t)items.size();
+    e->nsplit = nsplit;
     e->high_water = hw;
     e->max_small_n = 0;
     for (int32_t r = 0; r < R; ++r)
@@ -286,12 +331,14 @@ int rebuild(nb_engine* e) {
     return NB_OK;
 }
 
-nb::BatchForce force_args(nb_engine* e, const int2* items, int32_t nitems) {
+nb::BatchForce force_args(nb_engine* e, const nb::BatchItem* items, int32_t nitems, int32_t nsplit) {
     nb::BatchForce f{};
     f.sys = e->sysdesc;
     f.items = items;
     f.nitems = nitems;
+    f.nsplit = nsplit;
     f.counter = e->counter;
+    f.partial = e->partial;
     f.perm = e->lperm;
     f.pack = e->pack;
     f.origin = e->origin;
@@ -362,7 +409,7 @@ cudaError_t enqueue_step(nb_engine* e, cudaStream_t s, bool gated) {
     // force with the step's kick fused into its epilogue: every target of the
     // work items is a particle of a running system, and those are exactly
     // the particles the kick moves (fac_step 1)
-    nb::BatchForce f = force_args(e, e->items, e->nitems);
+    nb::BatchForce f = force_args(e, e->items, e->nitems, e->nsplit);
     f.vx = e->vx;
     f.vy = e->vy;
     f.vz = e->vz;
@@ -447,14 +494,16 @@ int start_systems(nb_engine* e, const std::vector<int32_t>& slots) {
     for (int32_t s : slots) ranks.push_back(ros[s]);
     std::stable_sort(ranks.begin(), ranks.end(),
                      [&](int32_t a, int32_t b) { return sd[a].ntiles > sd[b].ntiles; });
-    std::vector<int2> items;
-    for (int32_t r : ranks)
-        for (int32_t b = 0; b < sd[r].nblocks; ++b) items.push_back(make_int2(r, b));
-    NE_CK(cudaMemcpy(e->items_new, items.data(), sizeof(int2) * items.size(), cudaMemcpyHostToDevice));
+    std::vector<nb::BatchItem> items;
+    int64_t prow = 0;
+    int32_t nsplit = 0;
+    for (int32_t r : ranks) add_items(e, items, r, sd[r], prow, nsplit);
+    NE_CK(cudaMemcpy(e->items_new, items.data(), sizeof(nb::BatchItem) * items.size(),
+                     cudaMemcpyHostToDevice));
     // New systems have step count 0, so they are due for ordering; the others
     // keep their order (their schedule must not depend on admissions).
     NE_CK(enqueue_sort_pack(e, e->stream, false, false));
-    NE_CK(nb::launch_force_batch(e->p.law, force_args(e, e->items_new, (int32_t)items.size()),
+    NE_CK(nb::launch_force_batch(e->p.law, force_args(e, e->items_new, (int32_t)items.size(), nsplit),
                                  e->occ_acc * e->nsm, e->fblock, e->fipt, e->stream));
     return half_kick(e, slots, 0.5);
 }
@@ -629,10 +678,13 @@ int nb_engine_create(const nb_engine_params* p, nb_engine** out) {
     size_t o_dt = take(sizeof(double) * S), o_fs = take(sizeof(double) * S);
     size_t o_fo = take(sizeof(double) * S);
     size_t o_lr = take(sizeof(int32_t) * S), o_bk = take(sizeof(unsigned long long) * 6 * S);
-    // work items: at most one per i-block of the smallest block (128 targets) per system
-    e->item_cap = P / 128 + S;
-    size_t o_it = take(sizeof(int2) * (size_t)e->item_cap), o_itn = take(sizeof(int2) * (size_t)e->item_cap);
-    size_t o_cnt = take(sizeof(int32_t) * 4), o_err = take(sizeof(uint32_t) * 4);
+    // work items: blocks of at least 128 targets, a partial one per system, each in at most
+    // batch_max_parts() parts; the counter and one count per split block
+    const int64_t blocks = P / nb::batch_block_targets(e->fblock, e->fipt) + S;
+    e->item_cap = blocks * nb::batch_max_parts();
+    size_t o_it = take(sizeof(nb::BatchItem) * (size_t)e->item_cap);
+    size_t o_itn = take(sizeof(nb::BatchItem) * (size_t)e->item_cap);
+    size_t o_cnt = take(sizeof(int32_t) * (size_t)(1 + blocks)), o_err = take(sizeof(uint32_t) * 4);
     if (cudaMalloc(&e->arena, off) != cudaSuccess) {
         cudaStreamDestroy(e->stream);
         delete e;
@@ -660,8 +712,8 @@ int nb_engine_create(const nb_engine_params* p, nb_engine** out) {
     e->fac_once = (double*)(b + o_fo);
     e->large_ranks = (int32_t*)(b + o_lr);
     e->box_key = (unsigned long long*)(b + o_bk);
-    e->items = (int2*)(b + o_it);
-    e->items_new = (int2*)(b + o_itn);
+    e->items = (nb::BatchItem*)(b + o_it);
+    e->items_new = (nb::BatchItem*)(b + o_itn);
     e->counter = (int32_t*)(b + o_cnt);
     e->derr = (uint32_t*)(b + o_err);
     cudaMemset(e->derr, 0, sizeof(uint32_t));
@@ -689,6 +741,7 @@ int nb_engine_destroy(nb_engine* e) {
     drop_graph(e);
     if (e->ev0) cudaEventDestroy(e->ev0);
     if (e->ev1) cudaEventDestroy(e->ev1);
+    if (e->partial) cudaFree(e->partial);
     cudaFree(e->arena);
     cudaStreamDestroy(e->stream);
     delete e;

@@ -191,6 +191,19 @@ size_t worklist_partial_bytes(int64_t grid);
 int worklist_block_targets();
 
 // Many-system engine (nb_batch.cu, nb_engine.cu).
+// Work item of the batch force: i-block `block` of the system of rank `rank`,
+// over part `part` of `nparts` equal parts of the system's j-tiles.  The
+// partial sums of block b of a split system are kept from row prow on, one
+// row per part; the last part to finish joins them, counted at done.
+struct BatchItem {
+    int32_t rank;
+    int32_t block;
+    int32_t part;
+    int32_t nparts;
+    int32_t prow;
+    int32_t done;
+};
+
 struct BatchSys {
     int64_t aoff;  // first arena particle
     int64_t soff;  // first sorted slot
@@ -200,12 +213,13 @@ struct BatchSys {
 
 struct BatchForce {
     const SysDesc* sys;   // by rank; off = first sorted slot
-    const int2* items;    // (rank, i-block), largest systems first
+    const BatchItem* items;  // largest systems first
     // sys[r].off is the system's first arena particle and perm its
     // arena-relative Morton order: slot q is particle off + perm[off + q]
     int32_t nitems;
-    int32_t pad;
-    int32_t* counter;     // claim counter, zeroed by the launch
+    int32_t nsplit;       // blocks whose tiles are split
+    int32_t* counter;     // claim counter, then nsplit counts of finished parts; zeroed by the launch
+    float* partial;       // batch_partial_row() floats per (split block, part)
     const int32_t* perm;  // sorted slot -> arena particle
     const float4* pack;
     const TileOrigin* origin;
@@ -242,6 +256,11 @@ cudaError_t launch_fill_i32(int32_t* a, int64_t n, int32_t v, cudaStream_t s);
 int batch_ctas_per_sm(int law, bool acc, bool pot, int block, int ipt);
 bool batch_shape_ok(int block, int ipt);
 int batch_block_targets(int block, int ipt);
+// Parts that the j-tiles of a system of n particles are split into, and the
+// floats that a part's sums take.
+int batch_parts(int64_t n, int block, int ipt);
+int batch_max_parts();
+size_t batch_partial_row(int block, int ipt);
 // Morton order of the systems too large for the shared-memory sort ("large"
 // systems, listed by rank in ranks[0 .. nlarge)): their particles only, at
 // compact offsets BatchSys::soff (0 .. nl), are keyed (large index << 42 |
