@@ -31,13 +31,12 @@ struct LoopShape {
 constexpr uint64_t kWaitTimeoutNs = 2000000000ull;  // 2 s
 
 // ---------------------------------------------------------------------------
-// Spline slow path (r < h), FP32.  Returns m*fac (to multiply d) in mr3 and the
-// negated potential contribution in mp.
+// Spline slow path (0 <= r < h), FP32, with hinv = 1/h and hinv3 = hinv^3.
+// Returns m*fac (to multiply d) in mr3 and the negated potential contribution
+// in mp.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void spline_close(float r2, float rinv, float m, float h, float& mr3,
-                                             float& mp) {
-    const float hinv = 1.0f / h;
-    const float hinv3 = hinv * hinv * hinv;
+__device__ __forceinline__ void spline_close(float r2, float rinv, float m, float hinv, float hinv3,
+                                             float& mr3, float& mp) {
     const float r = (r2 > 0.0f) ? r2 * rinv : 0.0f;
     const float u = r * hinv;
     float fac, wp;
@@ -305,9 +304,8 @@ __device__ __forceinline__ void pair_loop_checked_impl(const float4* __restrict_
     // clamped to at least h^2: a pair with r < h adds the bounded Newtonian
     // term of distance h, m d / h^3 (the self pair, d = 0, adds no force),
     // and the smallest unclamped r^2 of every block of 8 source pairs marks
-    // the blocks that held such a pair.  Pass 2 revisits only the blocks that
-    // some lane of the warp flagged and replaces, for each r < h pair, the
-    // clamped term by the spline term.  Both terms are at most about m / h^2,
+    // the blocks that held such a pair.  Pass 2 revisits those blocks and
+    // replaces, for each r < h pair, the clamped term by the spline term.  Both terms are at most about m / h^2,
     // so the replacement loses nothing to cancellation.
     constexpr int NA = LoopShape<IPT>::NA;
     float2 nx[IPT], ny[IPT], nz[IPT], hc[IPT];
@@ -384,46 +382,58 @@ __device__ __forceinline__ void pair_loop_checked_impl(const float4* __restrict_
             tp[k] = __fmul2_rn(tp[k], m2);
         }
     }
-    for (uint32_t wb = __reduce_or_sync(0xffffffffu, blk); wb != 0u; wb &= wb - 1u) {
-        const int q0 = 8 * (__ffs(wb) - 1);
-#pragma unroll 1
-        for (int p = q0; p < q0 + 8; ++p) {
-            const float4 A = b[2 * p];
-            const float4 B = b[2 * p + 1];
-            const float2 qx = make_float2(A.x, A.y), qy = make_float2(A.z, A.w);
-            const float2 qz = make_float2(B.x, B.y), qm = make_float2(B.z, B.w);
+    // Pass 2, each lane over its own flagged blocks: it finds the block's r < h
+    // sources in a mask, then takes them one by one, in source order.  The warp
+    // waits for its lane with the most such sources.  (Walking the blocks that
+    // any lane flagged, pair by pair with a vote each, was a serial chain of
+    // some 130 cycles per pair: most of a small system's force time, since every
+    // target's own entry flags a block.)
+    // A pair with r = 0, every target's own entry among them, needs no
+    // correction of the force: both terms are d times a finite factor, d = 0.
+    // Only its potential term goes.
 #pragma unroll
-            for (int k = 0; k < IPT; ++k) {
-                const float2 dx = __fadd2_rn(qx, nx[k]);
-                const float2 dy = __fadd2_rn(qy, ny[k]);
-                const float2 dz = __fadd2_rn(qz, nz[k]);
+    for (int k = 0; k < IPT; ++k) {
+        if (blk == 0u) continue;
+        const float hinv = 1.0f / hh[k], hinv3 = hinv * hinv * hinv, rh = rsqrt_approx(h2[k]);
+        for (uint32_t m = blk; m != 0u; m &= m - 1u) {
+            const int q0 = 8 * (__ffs(m) - 1);
+            uint32_t hit = 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float4 A = b[2 * (q0 + i)];
+                const float4 B = b[2 * (q0 + i) + 1];
+                const float2 dx = __fadd2_rn(make_float2(A.x, A.y), nx[k]);
+                const float2 dy = __fadd2_rn(make_float2(A.z, A.w), ny[k]);
+                const float2 dz = __fadd2_rn(make_float2(B.x, B.y), nz[k]);
                 const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-                const bool cx = r2.x < h2[k], cy = r2.y < h2[k];
-                if (__any_sync(0xffffffffu, cx | cy)) {
-                    // the clamped Newtonian term pass 1 added: m r_h^-3 d and m r_h^-1
-                    const float rh = rsqrt_approx(h2[k]);
-                    if (cx) {
-                        const float m = UNI ? mu : qm.x;
-                        float mr3, mp;
-                        spline_close(r2.x, rsqrt_approx(r2.x), m, hh[k], mr3, mp);
-                        const float mrh = m * rh;
-                        const float d3 = mr3 - (mrh * rh) * rh;
-                        tx[k].x = fmaf(dx.x, d3, tx[k].x);
-                        ty[k].x = fmaf(dy.x, d3, ty[k].x);
-                        tz[k].x = fmaf(dz.x, d3, tz[k].x);
-                        tp[k].x += mp - mrh;
+                hit |= (uint32_t)(r2.x < h2[k] && (POT || r2.x > 0.0f)) << (2 * i);
+                hit |= (uint32_t)(r2.y < h2[k] && (POT || r2.y > 0.0f)) << (2 * i + 1);
+            }
+            for (; hit != 0u; hit &= hit - 1u) {
+                const int i = __ffs(hit) - 1, half = i & 1;
+                const float* f = reinterpret_cast<const float*>(b + 2 * (q0 + (i >> 1))) + half;
+                const float dx = f[0] + nx[k].x, dy = f[2] + ny[k].x, dz = f[4] + nz[k].x;
+                const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                const float mass = UNI ? mu : f[6];
+                float mr3, mp;
+                spline_close(r2, rsqrt_approx(r2), mass, hinv, hinv3, mr3, mp);
+                // minus the clamped Newtonian term of pass 1, m r_h^-3 d and m r_h^-1
+                const float mrh = mass * rh;
+                const float d3 = mr3 - (mrh * rh) * rh;
+                if (half == 0) {
+                    if (r2 > 0.0f) {
+                        tx[k].x = fmaf(dx, d3, tx[k].x);
+                        ty[k].x = fmaf(dy, d3, ty[k].x);
+                        tz[k].x = fmaf(dz, d3, tz[k].x);
                     }
-                    if (cy) {
-                        const float m = UNI ? mu : qm.y;
-                        float mr3, mp;
-                        spline_close(r2.y, rsqrt_approx(r2.y), m, hh[k], mr3, mp);
-                        const float mrh = m * rh;
-                        const float d3 = mr3 - (mrh * rh) * rh;
-                        tx[k].y = fmaf(dx.y, d3, tx[k].y);
-                        ty[k].y = fmaf(dy.y, d3, ty[k].y);
-                        tz[k].y = fmaf(dz.y, d3, tz[k].y);
-                        tp[k].y += mp - mrh;
+                    if (POT) tp[k].x += mp - mrh;
+                } else {
+                    if (r2 > 0.0f) {
+                        tx[k].y = fmaf(dx, d3, tx[k].y);
+                        ty[k].y = fmaf(dy, d3, ty[k].y);
+                        tz[k].y = fmaf(dz, d3, tz[k].y);
                     }
+                    if (POT) tp[k].y += mp - mrh;
                 }
             }
         }
