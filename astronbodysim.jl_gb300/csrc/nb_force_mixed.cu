@@ -8,27 +8,27 @@ extern template cudaError_t launch_force_mixed_tile<128>(int, bool, const Source
                                                          double, uint32_t*, int, int, int, cudaStream_t);
 extern template cudaError_t launch_pack_tile<128>(const double*, const double*, const double*,
                                                   const double*, int64_t, const int32_t*, float4*,
-                                                  TileOrigin*, float4*, cudaStream_t);
+                                                  TileOrigin*, float4*, const PackExtra&, cudaStream_t);
 extern template cudaError_t launch_force_mixed_tile<256>(int, bool, const Sources32&, const Targets&,
                                                          double, uint32_t*, int, int, int, cudaStream_t);
 extern template cudaError_t launch_pack_tile<256>(const double*, const double*, const double*,
                                                   const double*, int64_t, const int32_t*, float4*,
-                                                  TileOrigin*, float4*, cudaStream_t);
+                                                  TileOrigin*, float4*, const PackExtra&, cudaStream_t);
 extern template cudaError_t launch_force_mixed_tile<512>(int, bool, const Sources32&, const Targets&,
                                                          double, uint32_t*, int, int, int, cudaStream_t);
 extern template cudaError_t launch_pack_tile<512>(const double*, const double*, const double*,
                                                   const double*, int64_t, const int32_t*, float4*,
-                                                  TileOrigin*, float4*, cudaStream_t);
+                                                  TileOrigin*, float4*, const PackExtra&, cudaStream_t);
 
 bool tile_size_ok(int tile_j) { return tile_j == 128 || tile_j == 256 || tile_j == 512; }
 
 cudaError_t launch_pack(const double* x, const double* y, const double* z, const double* m,
                         int64_t n, const int32_t* perm, int tile_j, float4* pack,
-                        TileOrigin* origin, float4* ext, cudaStream_t s) {
+                        TileOrigin* origin, float4* ext, const PackExtra& px, cudaStream_t s) {
     switch (tile_j) {
-        case 128: return launch_pack_tile<128>(x, y, z, m, n, perm, pack, origin, ext, s);
-        case 256: return launch_pack_tile<256>(x, y, z, m, n, perm, pack, origin, ext, s);
-        case 512: return launch_pack_tile<512>(x, y, z, m, n, perm, pack, origin, ext, s);
+        case 128: return launch_pack_tile<128>(x, y, z, m, n, perm, pack, origin, ext, px, s);
+        case 256: return launch_pack_tile<256>(x, y, z, m, n, perm, pack, origin, ext, px, s);
+        case 512: return launch_pack_tile<512>(x, y, z, m, n, perm, pack, origin, ext, px, s);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -34,7 +34,13 @@ namespace nb {
 // origin is the centre of the tile's FP64 bounding box, origin.w its half
 // diagonal.
 // ---------------------------------------------------------------------------
-template <int TJ>
+// Optional extras (PackExtra): with DRIFT each particle takes its constant-step
+// drift first, in the operation order of k_drift (the step's own kernel for it
+// read and wrote the same positions once more); the split positions go out by
+// slot for the force kernel, which otherwise gathers and splits them anew in
+// every CTA (12 FP64-pipe operations per target, 0.4 us of an SM's FP64 pipe
+// per 128 targets).
+template <int TJ, bool DRIFT>
 __global__ void __launch_bounds__(TJ) k_pack(const double* __restrict__ x,
                                                  const double* __restrict__ y,
                                                  const double* __restrict__ z,
@@ -42,7 +48,7 @@ __global__ void __launch_bounds__(TJ) k_pack(const double* __restrict__ x,
                                                  const int32_t* __restrict__ perm,
                                                  float4* __restrict__ pack,
                                                  TileOrigin* __restrict__ origin,
-                                                 float4* __restrict__ ext) {
+                                                 float4* __restrict__ ext, PackExtra e) {
     // Each particle is split once into a double-float pair (12 FP64-pipe
     // operations, the slow pipe on this GPU).  The tile's box is reduced in
     // FP32 from the pairs relative to the tile's first particle c, the
@@ -55,14 +61,32 @@ __global__ void __launch_bounds__(TJ) k_pack(const double* __restrict__ x,
     const int64_t i = (int64_t)blockIdx.x * TJ + threadIdx.x;
     const bool valid = i < n;
     double px = 0.0, py = 0.0, pz = 0.0, pm = 0.0;
+    float hs = 0.0f;
+    if (e.done)
+        for (int64_t k = i; k < e.ndone; k += (int64_t)gridDim.x * TJ) e.done[k] = 0;
     if (valid) {
         const int64_t p = perm ? (int64_t)perm[i] : i;
-        px = x[p];
-        py = y[p];
-        pz = z[p];
+        if (DRIFT) {
+            const double t = e.clk->t_float, dt = __dadd_rn(__dadd_rn(t, e.dt), -t);
+            px = __dadd_rn(e.x[p], __dmul_rn(e.vx[p], dt));
+            py = __dadd_rn(e.y[p], __dmul_rn(e.vy[p], dt));
+            pz = __dadd_rn(e.z[p], __dmul_rn(e.vz[p], dt));
+            e.x[p] = px;
+            e.y[p] = py;
+            e.z[p] = pz;
+        } else {
+            px = x[p];
+            py = y[p];
+            pz = z[p];
+        }
         pm = m[p];
+        if (e.split) hs = (float)(e.type ? e.soft[e.type[p] - 1] : e.h_const);
     }
     const float2 sx = split_df(px), sy = split_df(py), sz = split_df(pz);
+    if (e.split && valid) {
+        e.split[2 * i] = make_float4(sx.x, sx.y, sy.x, sy.y);
+        e.split[2 * i + 1] = make_float4(sz.x, sz.y, hs, 0.0f);
+    }
     if (threadIdx.x == 0) {  // every tile holds at least one particle (tiles cover [0, n))
         cref[0] = px;
         cref[1] = py;
@@ -211,11 +235,12 @@ __global__ void __launch_bounds__(BLOCK, (ForceOcc<BLOCK, IPT, POT>::value)) k_f
     __shared__ float2 tpx[BLOCK * IPT], tpy[BLOCK * IPT], tpz[BLOCK * IPT];
 
     const int64_t ntg = tg.d_count ? (int64_t)(*tg.d_count) : tg.n;
-    const int js = src.jsplit > 1 ? src.jsplit : 1;
+    const int64_t nblk = (ntg + BLOCK * IPT - 1) / (BLOCK * IPT);
+    const int js = !src.partial ? 1 : src.jsplit > 0 ? src.jsplit : split_parts(nblk, src.ntiles);
     const int64_t blk = (int64_t)blockIdx.x / js;
     const int part = (int)(blockIdx.x % js);
     const int64_t base = blk * (BLOCK * IPT);
-    if (base >= ntg) return;  // CTA-uniform
+    if (blk >= nblk) return;  // CTA-uniform
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int t_lo = (int)((int64_t)part * src.ntiles / js);
@@ -231,12 +256,26 @@ __global__ void __launch_bounds__(BLOCK, (ForceOcc<BLOCK, IPT, POT>::value)) k_f
         fence_mbar_init();
     }
 
-    int32_t pidx[IPT];
+    int32_t pidx[IPT];  // the particle index, or with split positions the slot; -1: none
     float hh[IPT], h2[IPT];
 #pragma unroll
     for (int k = 0; k < IPT; ++k) {
         const int64_t t = base + k * BLOCK + tid;
         pidx[k] = -1;
+        if (tg.split) {
+            float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
+            if (t < ntg) {
+                pidx[k] = (int32_t)t;
+                a = tg.split[2 * t];
+                b = tg.split[2 * t + 1];
+            }
+            tpx[k * BLOCK + tid] = make_float2(a.x, a.y);
+            tpy[k * BLOCK + tid] = make_float2(a.z, a.w);
+            tpz[k * BLOCK + tid] = make_float2(b.x, b.y);
+            hh[k] = b.z;
+            h2[k] = hh[k] * hh[k];
+            continue;
+        }
         double x = 0.0, y = 0.0, z = 0.0, h = tg.h_const;
         if (t < ntg) {
             const int32_t p = tg.idx ? tg.idx[t] : (int32_t)t;
@@ -345,30 +384,98 @@ __global__ void __launch_bounds__(BLOCK, (ForceOcc<BLOCK, IPT, POT>::value)) k_f
     }
 
     if (js > 1) {
-        // j-split: compensated partials of this CTA's tile range
+        // Compensated partials of this CTA's tile range; the CTA that finishes
+        // last adds its block's parts in part order as double-float numbers in
+        // FP32 (TwoSum of the sums, carries added), about 48 bits.  Which CTA
+        // that is does not change the result.
+        constexpr int64_t kPer = BLOCK * IPT;
+        float* q0 = src.partial + blk * js * 8 * kPer + tid;
 #pragma unroll
         for (int k = 0; k < IPT; ++k) {
-            const int64_t slot = base + k * BLOCK + tid;
-            float* q = src.partial + (int64_t)part * 8 * src.pstride + slot;
-            q[0 * src.pstride] = sx[k];
-            q[1 * src.pstride] = cx[k];
-            q[2 * src.pstride] = sy[k];
-            q[3 * src.pstride] = cy[k];
-            q[4 * src.pstride] = sz[k];
-            q[5 * src.pstride] = cz[k];
-            q[6 * src.pstride] = sp[k];
-            q[7 * src.pstride] = cp[k];
+            float* q = q0 + part * 8 * kPer + k * BLOCK;
+            const float v[8] = {sx[k], cx[k], sy[k], cy[k], sz[k], cz[k], sp[k], cp[k]};
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (j < 6 ? ACC : POT) __stcg(q + j * kPer, v[j]);
         }
-        return;
+        __threadfence();  // the sums before the count
+        __syncthreads();
+        if (tid == 0) abort_flag = atomicAdd(&src.done[blk], 1u) == (uint32_t)(js - 1);
+        __syncthreads();
+        if (!abort_flag) return;
+        if (tg.vx) {  // the velocities that the kick will want
+#pragma unroll
+            for (int k = 0; k < IPT; ++k) {
+                if (pidx[k] < 0) continue;
+                const int32_t p = tg.split && tg.idx ? tg.idx[pidx[k]] : pidx[k];
+                prefetch_l1(tg.vx + p);
+                prefetch_l1(tg.vy + p);
+                prefetch_l1(tg.vz + p);
+            }
+        }
+        __threadfence();  // the count before the other parts' sums
+#pragma unroll
+        for (int k = 0; k < IPT; ++k) {
+            sx[k] = sy[k] = sz[k] = sp[k] = 0.0f;
+            cx[k] = cy[k] = cz[k] = cp[k] = 0.0f;
+        }
+        // kJU parts at a time, their loads in flight together (an L2 round trip
+        // each batch, which the join of a small system mostly waits for)
+        constexpr int kJU = IPT == 1 ? 8 : 4;
+#pragma unroll
+        for (int k = 0; k < IPT; ++k) {
+            for (int u0 = 0; u0 < js; u0 += kJU) {
+                float v[kJU][8];
+#pragma unroll
+                for (int u = 0; u < kJU; ++u)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (j < 6 ? ACC : POT)
+                            v[u][j] = u0 + u < js ? __ldcg(q0 + ((u0 + u) * 8 + j) * kPer + k * BLOCK) : 0.0f;
+#pragma unroll
+                for (int u = 0; u < kJU; ++u) {
+                    if (ACC) {
+                        two_sum_acc(sx[k], cx[k], v[u][0]);
+                        cx[k] += v[u][1];
+                        two_sum_acc(sy[k], cy[k], v[u][2]);
+                        cy[k] += v[u][3];
+                        two_sum_acc(sz[k], cz[k], v[u][4]);
+                        cz[k] += v[u][5];
+                    }
+                    if (POT) {
+                        two_sum_acc(sp[k], cp[k], v[u][6]);
+                        cp[k] += v[u][7];
+                    }
+                }
+            }
+        }
+    }
+    if (tg.step_clk && blk == 0 && tid == 0) {
+        // the clock update of a constant step whose drift ran in the pack
+        Clock* c = tg.step_clk;
+        const double t = c->t_float;
+        c->t_float = __dadd_rn(t, tg.kick_dt);
+        c->dt_drift = __dadd_rn(c->t_float, -t);
+        c->last_t_float = c->t_float;  // src/run.jl:164
+        c->interactions = __dadd_rn(c->interactions, __dmul_rn((double)tg.n, (double)tg.n));
+        c->steps += 1;
     }
 #pragma unroll
     for (int k = 0; k < IPT; ++k) {
-        const int32_t p = pidx[k];
-        if (p < 0) continue;
+        if (pidx[k] < 0) continue;
+        const int32_t p = tg.split && tg.idx ? tg.idx[pidx[k]] : pidx[k];
         if (ACC) {
-            tg.ax[p] = ((double)sx[k] + (double)cx[k]) * G;
-            tg.ay[p] = ((double)sy[k] + (double)cy[k]) * G;
-            tg.az[p] = ((double)sz[k] + (double)cz[k]) * G;
+            const double a0 = ((double)sx[k] + (double)cx[k]) * G;
+            const double a1 = ((double)sy[k] + (double)cy[k]) * G;
+            const double a2 = ((double)sz[k] + (double)cz[k]) * G;
+            tg.ax[p] = a0;
+            tg.ay[p] = a1;
+            tg.az[p] = a2;
+            if (tg.vx) {  // k_kick with constant steps, its operation order
+                tg.vx[p] = __dadd_rn(tg.vx[p], __dmul_rn(a0, tg.kick_dt));
+                tg.vy[p] = __dadd_rn(tg.vy[p], __dmul_rn(a1, tg.kick_dt));
+                tg.vz[p] = __dadd_rn(tg.vz[p], __dmul_rn(a2, tg.kick_dt));
+            }
         }
         if (POT) {
             // The loops accumulate +m/r; phi = -sum.
@@ -383,46 +490,6 @@ __global__ void __launch_bounds__(BLOCK, (ForceOcc<BLOCK, IPT, POT>::value)) k_f
     }
 }
 
-// Adds the j-split partials of every target in part order (deterministic).
-// The compensated (sum, carry) pairs of the parts are added as double-float
-// numbers in FP32 (TwoSum of the sums, carries added), about 48 bits, and
-// converted to FP64 once: the slow FP64 pipe then does two conversions and
-// one add per component instead of two per part.  CTAs of kJoinThreads spread
-// a small target set over many SMs.
-constexpr int kJoinThreads = 64;
-template <int LAW, bool ACC, bool POT>
-__global__ void __launch_bounds__(kJoinThreads) k_force_join(Sources32 src, Targets tg, double G) {
-    const int64_t ntg = tg.d_count ? (int64_t)(*tg.d_count) : tg.n;
-    const int64_t slot = (int64_t)blockIdx.x * kJoinThreads + threadIdx.x;
-    if (slot >= ntg) return;
-    const int32_t p = tg.idx ? tg.idx[slot] : (int32_t)slot;
-    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f}, c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    for (int part = 0; part < src.jsplit; ++part) {
-        const float* q = src.partial + (int64_t)part * 8 * src.pstride + slot;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            two_sum_acc(s[j], c[j], q[(2 * j) * src.pstride]);
-            c[j] += q[(2 * j + 1) * src.pstride];
-        }
-    }
-    double a[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) a[j] = (double)s[j] + (double)c[j];
-    if (ACC) {
-        tg.ax[p] = a[0] * G;
-        tg.ay[p] = a[1] * G;
-        tg.az[p] = a[2] * G;
-    }
-    if (POT) {
-        double phi = -a[3];
-        if (LAW == NB_LAW_PLUMMER && tg.self_mass) {
-            const float h = (float)(tg.type ? tg.soft[tg.type[p] - 1] : tg.h_const);
-            phi += (double)((float)tg.self_mass[p] * rsqrt_approx(h * h));
-        }
-        tg.pot[p] = phi * G;
-    }
-}
-
 // Launch of one force evaluation with tiles of TJ sources (instantiated in
 // nb_force_mixed_t<TJ>.cu).  Shapes: (128 | 256 threads) x (1 | 2 | 4 targets
 // per thread) with the default 4-stage ring; the acceleration-only form of
@@ -432,10 +499,16 @@ __global__ void __launch_bounds__(kJoinThreads) k_force_join(Sources32 src, Targ
 template <int LAW, bool ACC, bool POT, int TJ>
 cudaError_t launch_cfg_tile(const Sources32& src, const Targets& tg, double G, uint32_t* err,
                             int block, int ipt, int stages, cudaStream_t s) {
-    const int64_t per = (int64_t)block * ipt;
-    const int js = src.jsplit > 1 ? src.jsplit : 1;
-    const int64_t grid = (tg.n + per - 1) / per * js;
-    if (grid <= 0) return cudaSuccess;
+    const int64_t per = (int64_t)block * ipt, nblk = (tg.n + per - 1) / per;
+    if (nblk <= 0) return cudaSuccess;
+    // an active list may hold fewer blocks, split into more parts each: at most
+    // kSplitItems items where that is more than 8 per block
+    const int js = !src.partial ? 1 : src.jsplit > 0 ? src.jsplit : split_parts(nblk, src.ntiles);
+    int64_t grid = nblk * js;
+    if (src.partial && src.jsplit == 0 && tg.d_count) {
+        const int64_t most = nblk * src.ntiles < kSplitItems ? nblk * src.ntiles : kSplitItems;
+        if (grid < most) grid = most;
+    }
     bool launched = false;
 #define NB_LAUNCH(B, I, S)                                                                  \
     if (!launched && block == B && ipt == I) {                                             \
@@ -466,10 +539,6 @@ cudaError_t launch_cfg_tile(const Sources32& src, const Targets& tg, double G, u
     }
 #undef NB_LAUNCH
     if (!launched) return cudaErrorInvalidValue;
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess || js == 1) return e;
-    k_force_join<LAW, ACC, POT><<<(unsigned)((tg.n + kJoinThreads - 1) / kJoinThreads), kJoinThreads, 0, s>>>(
-        src, tg, G);
     return cudaGetLastError();
 }
 
@@ -492,10 +561,13 @@ cudaError_t launch_force_mixed_tile(int law, bool pot, const Sources32& src, con
 template <int TJ>
 cudaError_t launch_pack_tile(const double* x, const double* y, const double* z, const double* m,
                              int64_t n, const int32_t* perm, float4* pack, TileOrigin* origin,
-                             float4* ext, cudaStream_t s) {
+                             float4* ext, const PackExtra& px, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     const int64_t ntiles = (n + TJ - 1) / TJ;
-    k_pack<TJ><<<(unsigned)ntiles, TJ, 0, s>>>(x, y, z, m, n, perm, pack, origin, ext);
+    if (px.vx)
+        k_pack<TJ, true><<<(unsigned)ntiles, TJ, 0, s>>>(x, y, z, m, n, perm, pack, origin, ext, px);
+    else
+        k_pack<TJ, false><<<(unsigned)ntiles, TJ, 0, s>>>(x, y, z, m, n, perm, pack, origin, ext, px);
     return cudaGetLastError();
 }
 

@@ -8,6 +8,6 @@ template cudaError_t launch_force_mixed_tile<128>(int, bool, const Sources32&, c
                                                  uint32_t*, int, int, int, cudaStream_t);
 template cudaError_t launch_pack_tile<128>(const double*, const double*, const double*,
                                           const double*, int64_t, const int32_t*, float4*,
-                                          TileOrigin*, float4*, cudaStream_t);
+                                          TileOrigin*, float4*, const PackExtra&, cudaStream_t);
 
 }  // namespace nb

@@ -346,6 +346,27 @@ cudaError_t launch_drift(double* x, double* y, double* z, const double* vx, cons
     return cudaGetLastError();
 }
 
+// k_drift of a constant step whose clock update comes later (with the force):
+// the interval is (t + dt) - t of the clock as it stands.
+__global__ void k_drift_ahead(double* __restrict__ x, double* __restrict__ y,
+                              double* __restrict__ z, const double* __restrict__ vx,
+                              const double* __restrict__ vy, const double* __restrict__ vz,
+                              int64_t n, double dt_step, const Clock* __restrict__ clk) {
+    const int64_t i = (int64_t)blockIdx.x * kBlock + threadIdx.x;
+    if (i >= n) return;
+    const double t = clk->t_float, dt = (t + dt_step) - t;
+    x[i] = x[i] + vx[i] * dt;
+    y[i] = y[i] + vy[i] * dt;
+    z[i] = z[i] + vz[i] * dt;
+}
+
+cudaError_t launch_drift_ahead(double* x, double* y, double* z, const double* vx, const double* vy,
+                               const double* vz, int64_t n, double dt, const Clock* clk,
+                               cudaStream_t s) {
+    if (n > 0) k_drift_ahead<<<grid_for(n), kBlock, 0, s>>>(x, y, z, vx, vy, vz, n, dt, clk);
+    return cudaGetLastError();
+}
+
 // find_next_sync_point_and_drift with snapshots (src/base/Timestep.jl:197-215
 // constant, :224-245 adaptive), one event per graph replay (single thread).
 // The step ends at t_float + dt (constant) or at min_endstep (adaptive); while

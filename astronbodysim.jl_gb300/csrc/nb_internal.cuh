@@ -118,6 +118,38 @@ struct Targets {
     // Plummer law only: targets are also sources at the same FP32 position
     // (the self pair contributes -m/h to the potential and is removed).
     const double* self_mass;
+    // Positions and softening by slot as the pack left them (see PackExtra),
+    // when slot t is the particle of packed source t; nullptr: gather by idx.
+    const float4* split;
+    // Optional constant-step kick fused into the epilogue, v += a * kick_dt as
+    // k_kick rounds it (vx nullptr: none), with the step's clock update.
+    double* vx;
+    double* vy;
+    double* vz;
+    double kick_dt;
+    Clock* step_clk;
+};
+
+// What the pack does beside packing, all optional: the constant-step drift of
+// each particle before it is packed (vx set: x += v * ((t + dt) - t), t read
+// from the clock, which the force's epilogue advances), the targets' split
+// positions (split[2 i], split[2 i + 1] = (x.hi, x.lo, y.hi, y.lo),
+// (z.hi, z.lo, h, 0) of slot i), and the zeroed join counters of the force.
+struct PackExtra {
+    double* x;  // the packed particles' positions, written by the drift
+    double* y;
+    double* z;
+    const double* vx;
+    const double* vy;
+    const double* vz;
+    const Clock* clk;
+    double dt;
+    float4* split;
+    const int32_t* type;  // nullptr -> h_const
+    double soft[6];
+    double h_const;
+    uint32_t* done;
+    int32_t ndone;
 };
 
 // Packed FP32 sources for the mixed kernel: j-tiles of tile_j particles,
@@ -128,14 +160,34 @@ struct Sources32 {
     const float4* ext;  // per tile: half extents of the box (x, y, z) and half diagonal
     int32_t ntiles;
     int32_t tile_j;
-    // j-split: each i-block's tiles are shared by jsplit CTAs, which write
-    // compensated partials (partial[(part * 8 + q) * pstride + slot]) that
-    // k_force_join adds in part order.  jsplit 1: no partials.
+    // j-split: each i-block's tiles are shared by js CTAs, which write
+    // compensated partials, one row of 8 x (targets of a block) floats per
+    // (block, part); the part that finishes last (counted in done[block],
+    // zeroed by the pack) adds them in part order.  jsplit > 0 gives js; 0
+    // leaves it to split_parts() on the device's target count.  partial
+    // nullptr: no split.
     int32_t jsplit;
     int32_t pad;
     float* partial;
-    int64_t pstride;
+    uint32_t* done;
 };
+
+// Parts that the tiles of each of nblocks blocks of targets are split into.
+// Many blocks take 8 parts each; fewer take as many as make kSplitItems items,
+// 7 to 8 waves of the 760 to 912 CTAs that the GPU holds, so that the last wave
+// costs little (N = 65536: 1535, 1506 and 1472 us a step with 1216, 3040 and
+// 6080 items; N = 24593: 269, 253 and 249 us).  A part has at least two tiles
+// unless single tiles still make one wave: starting, counting and joining a
+// part costs about as much as one tile of a small system (N = 4096: 26.7 us a
+// step with one tile, 25.7 with two, 26.4 with four).
+constexpr int64_t kSplitItems = 6080, kSplitWave = 912;
+__host__ __device__ __forceinline__ int split_parts(int64_t nblocks, int64_t ntiles) {
+    int64_t js = nblocks > 0 ? kSplitItems / nblocks : 1;
+    if (js < 8) js = 8;
+    const int64_t most = nblocks * ntiles <= kSplitWave ? ntiles : (ntiles + 1) / 2;
+    if (js > most) js = most;
+    return js < 1 ? 1 : (int)js;
+}
 
 // FP64 sources.
 struct Sources64 {
@@ -302,7 +354,7 @@ cudaError_t launch_batch_kick(double* vx, double* vy, double* vz, const double* 
 // Launch helpers implemented in the .cu files.
 cudaError_t launch_pack(const double* x, const double* y, const double* z, const double* m,
                         int64_t n, const int32_t* perm, int tile_j, float4* pack,
-                        TileOrigin* origin, float4* ext, cudaStream_t s);
+                        TileOrigin* origin, float4* ext, const PackExtra& px, cudaStream_t s);
 // Morton-order permutation of the particles (nb_sort.cu); scratch of
 // sort_scratch_bytes(n) bytes.
 size_t sort_scratch_bytes(int64_t n);
@@ -365,6 +417,9 @@ cudaError_t launch_min_endstep(const int64_t* ti_end, int64_t n, int64_t time_ba
 cudaError_t launch_drift(double* x, double* y, double* z, const double* vx, const double* vy,
                          const double* vz, int64_t n, TimeCfg cfg, Clock* clk, int mode,
                          int64_t t_int_arg, double t_float_arg, cudaStream_t s);
+cudaError_t launch_drift_ahead(double* x, double* y, double* z, const double* vx, const double* vy,
+                               const double* vz, int64_t n, double dt, const Clock* clk,
+                               cudaStream_t s);
 cudaError_t launch_clock_end_step(Clock* clk, int adaptive, int64_t n, cudaStream_t s);
 // One event of find_next_sync_point_and_drift (src/base/Timestep.jl:197-245):
 // the clock advances to the next output time when it falls inside the step
@@ -445,6 +500,10 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
             "r"(smem_u32(dst)),
         "l"(src), "r"(bytes), "r"(smem_u32(bar))
         : "memory");
+}
+
+__device__ __forceinline__ void prefetch_l1(const void* p) {
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
 
 __device__ __forceinline__ float rsqrt_approx(float x) {

@@ -144,7 +144,7 @@ extern "C" int nb_force_noalloc(int64_t n, const double* x, const double* y, con
     // The error word is the only state that must start at zero.
     e = cudaMemsetAsync(err, 0, sizeof(uint32_t), s);
     if (e == cudaSuccess) e = nb::launch_morton_sort(x, y, z, n, sort_scratch, perm, s);
-    if (e == cudaSuccess) e = nb::launch_pack(x, y, z, m, n, perm, kTile, pack, origin, ext, s);
+    if (e == cudaSuccess) e = nb::launch_pack(x, y, z, m, n, perm, kTile, pack, origin, ext, nb::PackExtra{}, s);
     if (e == cudaSuccess) {
         nb::Sources32 src{pack, origin, ext, (int32_t)((n + kTile - 1) / kTile), kTile};
         nb::Targets tg{};
