@@ -7,10 +7,21 @@
 //
 //   1. FP64 bounding box of all particles (two-stage min/max, deterministic);
 //   2. 63-bit Morton key per particle (21 bits per axis over the box);
-//   3. stable LSD radix sort of (key, index), 8-bit digits, 8 passes:
-//      per-block digit histograms -> one exclusive scan -> stable scatter that
-//      ranks equal digits by (round, warp, lane) order.
+//   3. stable LSD radix sort of (key, index), 8-bit digits, 8 passes.
 // The result is a deterministic permutation for given positions.
+//
+// The sort of up to kClusterSortMax keys is bound by latency: as a chain of
+// kernels (histogram, scan, scatter per pass, 27 launches with the keys) it took
+// 125 us at N = 4096 and 200 us at N = 65536.  It runs instead as one cluster
+// of up to 16 CTAs whose shared memory holds all keys, passes separated by
+// hardware cluster barriers, digit counts and keys exchanged through
+// distributed shared memory (k_sort_cluster): 34 us at N = 4096, 107 us at
+// N = 65536, 173 us (277 as a chain) at N = 131072.  Larger sorts, bound by their
+// passes over memory, and GPUs without room for the cluster keep the chain:
+// per-block digit histograms -> one exclusive scan -> stable scatter that ranks
+// equal digits by (round, warp, lane) order.
+#include <cooperative_groups.h>
+
 #include "nb_internal.cuh"
 
 namespace nb {
@@ -21,7 +32,9 @@ constexpr int kSortTile = kSortThreads * kSortItems;
 constexpr int kRadixBits = 8;
 constexpr int kRadix = 1 << kRadixBits;
 constexpr int kWarps = kSortThreads / 32;
-constexpr int kBboxBlocks = 256;
+constexpr int kBboxBlocks = 64;
+constexpr int kBboxThreads = 512;
+constexpr int kMortonThreads = 64;  // small CTAs: the FP64 divisions of a small system over many SMs
 
 int64_t sort_blocks(int64_t n) { return (n + kSortTile - 1) / kSortTile; }
 int64_t scan_tmp_words(int64_t len);
@@ -32,8 +45,8 @@ size_t sort_scratch_bytes(int64_t n) {
     const int64_t nb = sort_blocks(n);
     auto al = [](size_t v) { return (v + 255) / 256 * 256; };
     return al(sizeof(uint64_t) * n) * 2 + al(sizeof(int32_t) * n) +
-           al(sizeof(uint32_t) * (size_t)kRadix * nb) + al(sizeof(double) * 6 * kBboxBlocks) +
-           al(sizeof(double) * 8) + al(sizeof(uint32_t) * (size_t)scan_tmp_words(kRadix * nb));
+           al(sizeof(uint32_t) * (size_t)kRadix * nb) +
+           al(sizeof(unsigned long long) * 6 * kBboxBlocks) + al(sizeof(uint32_t) * (size_t)scan_tmp_words(kRadix * nb));
 }
 
 struct SortScratch {
@@ -41,8 +54,7 @@ struct SortScratch {
     uint64_t* keys_b;
     int32_t* vals_b;
     uint32_t* counts;
-    double* bbox_part;
-    double* bbox;
+    unsigned long long* bbox_part;
     uint32_t* scan_tmp;
 };
 
@@ -58,49 +70,55 @@ static SortScratch carve(void* base, int64_t n) {
     p += al(sizeof(int32_t) * n);
     s.counts = (uint32_t*)p;
     p += al(sizeof(uint32_t) * (size_t)kRadix * sort_blocks(n));
-    s.bbox_part = (double*)p;
-    p += al(sizeof(double) * 6 * kBboxBlocks);
-    s.bbox = (double*)p;
-    p += al(sizeof(double) * 8);
+    s.bbox_part = (unsigned long long*)p;
+    p += al(sizeof(unsigned long long) * 6 * kBboxBlocks);
     s.scan_tmp = (uint32_t*)p;
     return s;
 }
 
-__global__ void __launch_bounds__(kSortThreads)
-    k_bbox_partial(const double* __restrict__ x, const double* __restrict__ y,
-                   const double* __restrict__ z, int64_t n, double* __restrict__ part) {
-    __shared__ double red[6][kWarps];
-    double v[6] = {1e300, 1e300, 1e300, 1e300, 1e300, 1e300};  // min x,y,z and min -x,-y,-z
-    for (int64_t i = (int64_t)blockIdx.x * kSortThreads + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * kSortThreads) {
-        const double a = x[i], b = y[i], c = z[i];
-        v[0] = fmin(v[0], a);
-        v[1] = fmin(v[1], b);
-        v[2] = fmin(v[2], c);
-        v[3] = fmin(v[3], -a);
-        v[4] = fmin(v[4], -b);
-        v[5] = fmin(v[5], -c);
-    }
+// Order-preserving unsigned image of a double; a NaN never wins the minimum.
+// The box is reduced on these images, off the slow FP64 pipe.
+__device__ __forceinline__ unsigned long long ord_image(double v) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    return v != v ? ~0ull : (b >> 63) ? ~b : (b | 0x8000000000000000ull);
+}
+__device__ __forceinline__ double ord_double(unsigned long long k) {
+    return __longlong_as_double((long long)((k >> 63) ? (k & 0x7fffffffffffffffull) : ~k));
+}
+// The warp's minima of v[0..5].
+__device__ __forceinline__ void warp_min6(unsigned long long* v) {
 #pragma unroll
     for (int k = 0; k < 6; ++k)
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[k] = fmin(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
+        for (int o = 16; o > 0; o >>= 1) v[k] = min(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
+}
+
+// Minima of x, y, z, -x, -y, -z over each block's particles, as images.
+__global__ void __launch_bounds__(kBboxThreads)
+    k_bbox_partial(const double* __restrict__ x, const double* __restrict__ y,
+                   const double* __restrict__ z, int64_t n, unsigned long long* __restrict__ part) {
+    __shared__ unsigned long long red[6][kBboxThreads / 32];
+    const unsigned long long big = ord_image(1e300);
+    unsigned long long v[6] = {big, big, big, big, big, big};
+    for (int64_t i = (int64_t)blockIdx.x * kBboxThreads + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * kBboxThreads) {
+        const double a = x[i], b = y[i], c = z[i];
+        v[0] = min(v[0], ord_image(a));
+        v[1] = min(v[1], ord_image(b));
+        v[2] = min(v[2], ord_image(c));
+        v[3] = min(v[3], ord_image(-a));
+        v[4] = min(v[4], ord_image(-b));
+        v[5] = min(v[5], ord_image(-c));
+    }
+    warp_min6(v);
     if ((threadIdx.x & 31) == 0)
 #pragma unroll
         for (int k = 0; k < 6; ++k) red[k][threadIdx.x >> 5] = v[k];
     __syncthreads();
     if (threadIdx.x < 6) {
-        double r = red[threadIdx.x][0];
-        for (int w = 1; w < kWarps; ++w) r = fmin(r, red[threadIdx.x][w]);
+        unsigned long long r = red[threadIdx.x][0];
+        for (int w = 1; w < kBboxThreads / 32; ++w) r = min(r, red[threadIdx.x][w]);
         part[blockIdx.x * 6 + threadIdx.x] = r;
-    }
-}
-
-__global__ void k_bbox_final(const double* __restrict__ part, int nblocks, double* __restrict__ bbox) {
-    if (threadIdx.x < 6) {
-        double r = part[threadIdx.x];
-        for (int b = 1; b < nblocks; ++b) r = fmin(r, part[b * 6 + threadIdx.x]);
-        bbox[threadIdx.x] = r;  // lo[0..2] = r[0..2], hi[k] = -r[3+k]
     }
 }
 
@@ -114,13 +132,31 @@ __device__ __forceinline__ uint64_t spread3_21(uint64_t v) {
     return v;
 }
 
-__global__ void k_morton(const double* __restrict__ x, const double* __restrict__ y,
-                         const double* __restrict__ z, int64_t n, const double* __restrict__ bbox,
-                         uint64_t* __restrict__ keys, int32_t* __restrict__ vals) {
-    const int64_t i = (int64_t)blockIdx.x * kSortThreads + threadIdx.x;
+// Keys of all particles; every block joins the nblocks partial boxes for itself.
+__global__ void __launch_bounds__(kMortonThreads)
+    k_morton(const double* __restrict__ x, const double* __restrict__ y,
+             const double* __restrict__ z, int64_t n, const unsigned long long* __restrict__ part,
+             int nblocks, uint64_t* __restrict__ keys, int32_t* __restrict__ vals) {
+    __shared__ unsigned long long red[6][kMortonThreads / 32];
+    const unsigned long long big = ord_image(1e300);
+    unsigned long long v[6] = {big, big, big, big, big, big};
+    for (int b = threadIdx.x; b < nblocks; b += kMortonThreads)
+#pragma unroll
+        for (int k = 0; k < 6; ++k) v[k] = min(v[k], part[b * 6 + k]);
+    warp_min6(v);
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+        for (int k = 0; k < 6; ++k) red[k][threadIdx.x >> 5] = v[k];
+    __syncthreads();
+    const int64_t i = (int64_t)blockIdx.x * kMortonThreads + threadIdx.x;
     if (i >= n) return;
-    const double lo[3] = {bbox[0], bbox[1], bbox[2]};
-    const double hi[3] = {-bbox[3], -bbox[4], -bbox[5]};
+    double lo[3], hi[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        lo[k] = ord_double(min(red[k][0], red[k][1]));
+        hi[k] = -ord_double(min(red[k + 3][0], red[k + 3][1]));
+    }
+    static_assert(kMortonThreads == 64, "two warps' minima");
     const double p[3] = {x[i], y[i], z[i]};
     uint64_t q[3];
 #pragma unroll
@@ -306,6 +342,175 @@ cudaError_t launch_exclusive_scan(uint32_t* counts, int64_t len, cudaStream_t s)
     return cudaGetLastError();
 }
 
+// ---------------------------------------------------------------------------
+// Radix sort in one cluster.  CTA c of C holds positions [c M, (c + 1) M) of
+// the current order, M = kCsThreads * ITEMS, in shared memory (keys and values,
+// double-buffered).  A pass:
+//   * every warp ranks its 32 * ITEMS consecutive keys by digit, in order
+//     (match_any per round, running counts per warp and digit), and the CTA
+//     turns the warps' counts into offsets and publishes its digit counts;
+//   * after a cluster barrier each CTA reads all CTAs' counts, which gives
+//     the first position of each of its digits in the whole order;
+//   * keys and values go to their positions in the other buffer of the CTA
+//     that owns them (distributed shared memory); cluster barrier.
+// Stable, so the permutation is the same as that of the chain of kernels.
+// Positions past n are not stored; only the last CTAs have such.
+// ---------------------------------------------------------------------------
+constexpr int kCsThreads = 512;
+constexpr int kCsWarps = kCsThreads / 32;
+constexpr int kCsMaxItems = 16;
+constexpr int kCsMaxCluster = 16;
+constexpr int64_t kClusterSortMax = (int64_t)kCsMaxCluster * kCsThreads * kCsMaxItems;
+
+template <int ITEMS>
+struct CsShared {
+    uint64_t key[2][kCsThreads * ITEMS];
+    int32_t val[2][kCsThreads * ITEMS];
+    uint32_t cnt[kCsWarps][kRadix];  // per warp: counts, then offsets within the CTA
+    uint32_t total[kRadix];          // this CTA's digit counts, read by the others
+    uint32_t base[kRadix];           // first position of each of its digits
+    uint32_t wsum[kRadix / 32];
+};
+
+template <int ITEMS>
+__global__ void __launch_bounds__(kCsThreads)
+    k_sort_cluster(const uint64_t* __restrict__ keys, int32_t* __restrict__ vals, int n, int passes) {
+    namespace cg = cooperative_groups;
+    extern __shared__ __align__(16) unsigned char cs_raw[];
+    CsShared<ITEMS>& sh = *reinterpret_cast<CsShared<ITEMS>*>(cs_raw);
+    cg::cluster_group cluster = cg::this_cluster();
+    constexpr int M = kCsThreads * ITEMS;
+    const int C = (int)cluster.num_blocks(), c = (int)cluster.block_rank();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int first = c * M, count = min(M, max(0, n - first));  // keys this CTA holds
+    for (int i = tid; i < count; i += kCsThreads) {
+        sh.key[0][i] = keys[first + i];
+        sh.val[0][i] = vals[first + i];
+    }
+    // every CTA of the cluster runs before any of them writes into another
+    cluster.sync();
+    for (int pass = 0; pass < passes; ++pass) {
+        const int src = pass & 1, shift = pass * kRadixBits;
+        for (int d = lane; d < kRadix; d += 32) sh.cnt[warp][d] = 0;
+        __syncwarp();
+        uint64_t key[ITEMS];
+        uint32_t rank[ITEMS];
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r) {
+            const int i = warp * 32 * ITEMS + r * 32 + lane;
+            const bool valid = i < count;
+            key[r] = valid ? sh.key[src][i] : 0ull;
+            const uint32_t d = valid ? (uint32_t)(key[r] >> shift) & (kRadix - 1) : (uint32_t)kRadix;
+            const uint32_t peers = __match_any_sync(0xffffffffu, d);
+            const uint32_t before = __popc(peers & ((1u << lane) - 1u));
+            rank[r] = valid ? sh.cnt[warp][d] + before : 0u;
+            __syncwarp();
+            if (valid && before == 0u) sh.cnt[warp][d] += __popc(peers);
+            __syncwarp();
+        }
+        __syncthreads();
+        if (tid < kRadix) {
+            uint32_t run = 0;
+#pragma unroll
+            for (int w = 0; w < kCsWarps; ++w) {
+                const uint32_t v = sh.cnt[w][tid];
+                sh.cnt[w][tid] = run;
+                run += v;
+            }
+            sh.total[tid] = run;
+        }
+        cluster.sync();
+        uint32_t all = 0, prev = 0, incl = 0;
+        if (tid < kRadix) {
+#pragma unroll 8
+            for (int k = 0; k < C; ++k) {
+                const uint32_t v = *cluster.map_shared_rank(&sh.total[tid], k);
+                all += v;
+                prev += k < c ? v : 0u;
+            }
+            incl = all;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            if (lane == 31) sh.wsum[warp] = incl;
+        }
+        __syncthreads();
+        if (tid < kRadix) {
+            uint32_t b = incl - all + prev;
+            for (int w = 0; w < warp; ++w) b += sh.wsum[w];
+            sh.base[tid] = b;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r) {
+            const int i = warp * 32 * ITEMS + r * 32 + lane;
+            if (i < count) {
+                const uint32_t d = (uint32_t)(key[r] >> shift) & (kRadix - 1);
+                const uint32_t pos = sh.base[d] + sh.cnt[warp][d] + rank[r];
+                const int to = (int)(pos / M), at = (int)(pos % M);
+                *cluster.map_shared_rank(&sh.key[src ^ 1][at], to) = key[r];
+                *cluster.map_shared_rank(&sh.val[src ^ 1][at], to) = sh.val[src][i];
+            }
+        }
+        // all keys have arrived; also the last read of total, and of a CTA's
+        // shared memory by another, before it is written again or given up
+        cluster.sync();
+    }
+    for (int i = tid; i < count; i += kCsThreads) vals[first + i] = sh.val[passes & 1][i];
+}
+
+// Launches the cluster sort of n <= C * kCsThreads * ITEMS keys; *done false:
+// this GPU cannot hold the cluster (nothing was launched).
+template <int ITEMS>
+static cudaError_t launch_cluster(const uint64_t* keys, int32_t* vals, int64_t n, int passes, bool* done,
+                                  cudaStream_t s) {
+    auto kern = k_sort_cluster<ITEMS>;
+    constexpr size_t smem = sizeof(CsShared<ITEMS>);
+    static_assert(smem <= 232448, "227 KB of shared memory per CTA");
+    int C = 1;
+    while ((int64_t)C * kCsThreads * ITEMS < n) C *= 2;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess && C > 8)
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)C);
+    cfg.blockDim = dim3(kCsThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)C;
+    at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg);
+    if (e != cudaSuccess || clusters < 1) {
+        (void)cudaGetLastError();
+        *done = false;
+        return cudaSuccess;
+    }
+    *done = true;
+    return cudaLaunchKernelEx(&cfg, kern, keys, vals, (int)n, passes);
+}
+
+// As many CTAs as give each at least kCsThreads keys, up to the 16 of a
+// cluster, then more keys per thread.
+static cudaError_t launch_cluster_sort(const uint64_t* keys, int32_t* vals, int64_t n, int passes,
+                                       bool* done, cudaStream_t s) {
+    *done = false;
+    if (n > kClusterSortMax) return cudaSuccess;
+    const int64_t per = (n + kCsMaxCluster * kCsThreads - 1) / (kCsMaxCluster * kCsThreads);
+    if (per <= 1) return launch_cluster<1>(keys, vals, n, passes, done, s);
+    if (per <= 2) return launch_cluster<2>(keys, vals, n, passes, done, s);
+    if (per <= 4) return launch_cluster<4>(keys, vals, n, passes, done, s);
+    if (per <= 8) return launch_cluster<8>(keys, vals, n, passes, done, s);
+    return launch_cluster<16>(keys, vals, n, passes, done, s);
+}
+
 // Key buffer inside a sort scratch of sort_scratch_bytes(n) bytes.
 uint64_t* sort_keys_buffer(void* scratch, int64_t n) { return carve(scratch, n).keys_a; }
 
@@ -314,8 +519,10 @@ uint64_t* sort_keys_buffer(void* scratch, int64_t n) { return carve(scratch, n).
 cudaError_t launch_sort_keys(void* scratch, int64_t n, int32_t* vals, int passes, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     SortScratch sc = carve(scratch, n);
+    bool done = false;
+    cudaError_t e = launch_cluster_sort(sc.keys_a, vals, n, passes, &done, s);
+    if (e != cudaSuccess || done) return e;
     const int nblocks = (int)sort_blocks(n);
-    cudaError_t e = cudaSuccess;
     uint64_t* kin = sc.keys_a;
     uint64_t* kout = sc.keys_b;
     int32_t* vin = vals;
@@ -343,11 +550,11 @@ cudaError_t launch_morton_sort(const double* x, const double* y, const double* z
                                void* scratch, int32_t* perm, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     SortScratch sc = carve(scratch, n);
-    int64_t gb = (n + kSortThreads - 1) / kSortThreads;
+    const int64_t gb = (n + kBboxThreads - 1) / kBboxThreads;
     const int bb = (int)(gb < kBboxBlocks ? gb : kBboxBlocks);
-    k_bbox_partial<<<bb, kSortThreads, 0, s>>>(x, y, z, n, sc.bbox_part);
-    k_bbox_final<<<1, 32, 0, s>>>(sc.bbox_part, bb, sc.bbox);
-    k_morton<<<(unsigned)gb, kSortThreads, 0, s>>>(x, y, z, n, sc.bbox, sc.keys_a, perm);
+    k_bbox_partial<<<bb, kBboxThreads, 0, s>>>(x, y, z, n, sc.bbox_part);
+    k_morton<<<(unsigned)((n + kMortonThreads - 1) / kMortonThreads), kMortonThreads, 0, s>>>(
+        x, y, z, n, sc.bbox_part, bb, sc.keys_a, perm);
     return launch_sort_keys(scratch, n, perm, 8, s);
 }
 
