@@ -40,6 +40,13 @@ constexpr int kTile = 256;
 #define NB_ENGINE_RESORT_EVERY 64
 #endif
 constexpr int kResortEvery = NB_ENGINE_RESORT_EVERY;
+// Staging of batched admissions and retirements, on the device and in pinned
+// host memory: allocated with the first batch, freed with the engine.  A table
+// of kStageMoves systems, then their particles.
+constexpr int32_t kStageMoves = 1024;
+constexpr size_t kStageTable = sizeof(nb::BatchMove) * kStageMoves;
+constexpr size_t kStageBytes = (size_t)8 << 20;
+constexpr int64_t kStageDoubles = (int64_t)((kStageBytes - kStageTable) / sizeof(double));
 
 struct Request {
     int64_t id = 0;
@@ -97,6 +104,9 @@ struct nb_engine {
     // to what the running systems need, freed with the engine
     float* partial = nullptr;
     size_t partial_floats = 0;
+    void* stage = nullptr;   // device staging buffer, kStageBytes
+    void* hstage = nullptr;  // its pinned host copy
+    bool stage_failed = false;
     bool split = true;  // false: no memory for the partial sums, whole i-blocks instead
     uint32_t* derr = nullptr;
     int64_t tile_cap = 0;
@@ -423,54 +433,140 @@ cudaError_t enqueue_step(nb_engine* e, cudaStream_t s, bool gated) {
     return nb::launch_batch_tick(e->batchsys, e->nrank, e->steps_slot, nsteps, s);
 }
 
+nb::BatchArrays arena_arrays(nb_engine* e) {
+    return nb::BatchArrays{e->x,  e->y,  e->z,  e->vx, e->vy,    e->vz,
+                           e->m,  e->ax, e->ay, e->az, e->sysid, e->steps_slot};
+}
+
+// The staging buffers; false when there is no memory for them (systems then
+// move one at a time).
+bool have_stage(nb_engine* e) {
+    if (e->stage) return true;
+    if (e->stage_failed) return false;
+    if (cudaMalloc(&e->stage, kStageBytes) != cudaSuccess) e->stage = nullptr;
+    if (e->stage && cudaHostAlloc(&e->hstage, kStageBytes, cudaHostAllocDefault) != cudaSuccess) {
+        cudaFree(e->stage);
+        e->stage = nullptr;
+    }
+    if (!e->stage) {
+        (void)cudaGetLastError();
+        e->hstage = nullptr;
+        e->stage_failed = true;
+    }
+    return e->stage != nullptr;
+}
+
+// Systems that move through the staging buffer together.
+struct MoveBatch {
+    std::vector<nb::BatchMove> rows;
+    std::vector<Request*> reqs;
+    int64_t doubles = 0;
+    int32_t max_n = 0;
+
+    bool fits(int64_t d) const { return (int32_t)rows.size() < kStageMoves && doubles + d <= kStageDoubles; }
+    void add(Request* q, int64_t aoff, int32_t slot, int64_t d) {
+        rows.push_back(nb::BatchMove{doubles, aoff, (int32_t)q->n, slot});
+        reqs.push_back(q);
+        doubles += d;
+        max_n = std::max(max_n, (int32_t)q->n);
+    }
+    void clear() {
+        rows.clear();
+        reqs.clear();
+        doubles = 0;
+        max_n = 0;
+    }
+};
+
+// Device addresses of the staged table and particles.
+nb::BatchMove* stage_table(nb_engine* e) { return static_cast<nb::BatchMove*>(e->stage); }
+double* stage_data(nb_engine* e) {
+    return reinterpret_cast<double*>(static_cast<char*>(e->stage) + kStageTable);
+}
+char* hstage_data(nb_engine* e) { return static_cast<char*>(e->hstage) + kStageTable; }
+
+int flush_admissions(nb_engine* e, MoveBatch& b) {
+    if (b.rows.empty()) return NB_OK;
+    std::memcpy(e->hstage, b.rows.data(), sizeof(nb::BatchMove) * b.rows.size());
+    for (size_t k = 0; k < b.rows.size(); ++k) {
+        Request& q = *b.reqs[k];
+        std::memcpy(hstage_data(e) + sizeof(double) * (size_t)b.rows[k].src, q.in.data(),
+                    sizeof(double) * 7 * (size_t)q.n);
+        q.in.clear();
+        q.in.shrink_to_fit();
+    }
+    NE_CK(cudaMemcpyAsync(e->stage, e->hstage, kStageTable + sizeof(double) * (size_t)b.doubles,
+                          cudaMemcpyHostToDevice, e->stream));
+    NE_CK(nb::launch_batch_admit(stage_table(e), (int32_t)b.rows.size(), b.max_n, stage_data(e),
+                                 arena_arrays(e), e->stream));
+    NE_CK(cudaStreamSynchronize(e->stream));  // before the staging buffer is filled again
+    b.clear();
+    return NB_OK;
+}
+
+// Copies one system into its arena range with copies of its own (systems
+// larger than the staging buffer, resumed ones).
+int admit_alone(nb_engine* e, Request& q, int64_t off, int32_t slot) {
+    const size_t d = sizeof(double) * (size_t)q.n;
+    const double* in = q.in.data();
+    double* dst[10] = {e->x, e->y, e->z, e->vx, e->vy, e->vz, e->m, e->ax, e->ay, e->az};
+    const int narr = q.resumed ? 10 : 7;
+    for (int k = 0; k < narr; ++k)
+        NE_CK(cudaMemcpyAsync(dst[k] + off, in + (size_t)k * q.n, d, cudaMemcpyHostToDevice, e->stream));
+    if (q.resumed) {
+        // own Morton order and step count, so the re-ordering schedule continues
+        NE_CK(cudaMemcpyAsync(e->lperm + off, q.order.data(), sizeof(int32_t) * (size_t)q.n,
+                              cudaMemcpyHostToDevice, e->stream));
+        NE_CK(cudaMemcpyAsync(e->steps_slot + slot, &q.steps_done, sizeof(int64_t),
+                              cudaMemcpyHostToDevice, e->stream));
+    } else {
+        NE_CK(cudaMemsetAsync(e->ax + off, 0, d, e->stream));
+        NE_CK(cudaMemsetAsync(e->ay + off, 0, d, e->stream));
+        NE_CK(cudaMemsetAsync(e->az + off, 0, d, e->stream));
+        NE_CK(cudaMemsetAsync(e->steps_slot + slot, 0, sizeof(int64_t), e->stream));
+    }
+    NE_CK(nb::launch_fill_i32(e->sysid + off, q.n, slot, e->stream));
+    NE_CK(cudaStreamSynchronize(e->stream));
+    q.in.clear();
+    q.in.shrink_to_fit();
+    q.order.clear();
+    q.order.shrink_to_fit();
+    return NB_OK;
+}
+
 // Admit queued requests (FIFO) while a slot and a particle range are free;
 // returns the slots admitted.
 int admit(nb_engine* e, std::vector<int32_t>& admitted) {
+    MoveBatch batch;
+    int32_t s0 = 0;  // slots before it are taken
     while (!e->queue.empty()) {
         Request& q = e->reqs[e->queue.front()];
-        int32_t slot = -1;
-        for (int32_t s = 0; s < (int32_t)e->slot_req.size(); ++s)
-            if (e->slot_req[s] < 0) {
-                slot = s;
-                break;
-            }
-        if (slot < 0) break;
+        while (s0 < (int32_t)e->slot_req.size() && e->slot_req[s0] >= 0) ++s0;
+        if (s0 == (int32_t)e->slot_req.size()) break;
+        const int32_t slot = s0;
         const int64_t off = alloc_range(e, q.n);
         if (off < 0) break;  // head of the queue waits for space (FIFO)
-        const size_t d = sizeof(double) * (size_t)q.n;
-        const double* in = q.in.data();
-        double* dst[10] = {e->x, e->y, e->z, e->vx, e->vy, e->vz, e->m, e->ax, e->ay, e->az};
-        const int narr = q.resumed ? 10 : 7;
-        for (int k = 0; k < narr; ++k)
-            NE_CK(cudaMemcpyAsync(dst[k] + off, in + (size_t)k * q.n, d, cudaMemcpyHostToDevice, e->stream));
-        if (q.resumed) {
-            // own Morton order and step count, so the re-ordering schedule continues
-            NE_CK(cudaMemcpyAsync(e->lperm + off, q.order.data(), sizeof(int32_t) * (size_t)q.n,
-                                  cudaMemcpyHostToDevice, e->stream));
-            NE_CK(cudaMemcpyAsync(e->steps_slot + slot, &q.steps_done, sizeof(int64_t),
-                                  cudaMemcpyHostToDevice, e->stream));
+        const int64_t doubles = 7 * q.n;
+        if (!q.resumed && doubles <= kStageDoubles && have_stage(e)) {
+            if (!batch.fits(doubles)) {
+                int rc = flush_admissions(e, batch);
+                if (rc) return rc;
+            }
+            batch.add(&q, off, slot, doubles);
         } else {
-            NE_CK(cudaMemsetAsync(e->ax + off, 0, d, e->stream));
-            NE_CK(cudaMemsetAsync(e->ay + off, 0, d, e->stream));
-            NE_CK(cudaMemsetAsync(e->az + off, 0, d, e->stream));
-            NE_CK(cudaMemsetAsync(e->steps_slot + slot, 0, sizeof(int64_t), e->stream));
+            int rc = admit_alone(e, q, off, slot);
+            if (rc) return rc;
         }
-        NE_CK(nb::launch_fill_i32(e->sysid + off, q.n, slot, e->stream));
-        NE_CK(cudaStreamSynchronize(e->stream));
         q.aoff = off;
         q.slot = slot;
         q.state = NB_REQ_RUNNING;
-        q.in.clear();
-        q.in.shrink_to_fit();
-        q.order.clear();
-        q.order.shrink_to_fit();
         e->slot_req[slot] = q.id;
         e->queue.pop_front();
         if (!q.resumed) admitted.push_back(slot);  // a resumed system needs no start-up
         q.resumed = false;
         e->dirty = true;
     }
-    return NB_OK;
+    return flush_admissions(e, batch);
 }
 
 // Kick the given slots by fac (+0.5 on admission, -0.5 on retirement).
@@ -508,6 +604,25 @@ int start_systems(nb_engine* e, const std::vector<int32_t>& slots) {
     return half_kick(e, slots, 0.5);
 }
 
+int flush_retirements(nb_engine* e, MoveBatch& b) {
+    if (b.rows.empty()) return NB_OK;
+    std::memcpy(e->hstage, b.rows.data(), sizeof(nb::BatchMove) * b.rows.size());
+    NE_CK(cudaMemcpyAsync(e->stage, e->hstage, sizeof(nb::BatchMove) * b.rows.size(),
+                          cudaMemcpyHostToDevice, e->stream));
+    NE_CK(nb::launch_batch_retire(stage_table(e), (int32_t)b.rows.size(), b.max_n, stage_data(e),
+                                  arena_arrays(e), e->stream));
+    NE_CK(cudaMemcpyAsync(hstage_data(e), stage_data(e), sizeof(double) * (size_t)b.doubles,
+                          cudaMemcpyDeviceToHost, e->stream));
+    NE_CK(cudaStreamSynchronize(e->stream));
+    for (size_t k = 0; k < b.rows.size(); ++k) {
+        Request& q = *b.reqs[k];
+        std::memcpy(q.out.data(), hstage_data(e) + sizeof(double) * (size_t)b.rows[k].src,
+                    sizeof(double) * 6 * (size_t)q.n);
+    }
+    b.clear();
+    return NB_OK;
+}
+
 // Retire systems whose step count is reached: -1/2 kick, download, free.
 int retire(nb_engine* e) {
     std::vector<int32_t> fin;
@@ -519,9 +634,19 @@ int retire(nb_engine* e) {
     if (fin.empty()) return NB_OK;
     int rc = half_kick(e, fin, -0.5);
     if (rc) return rc;
+    MoveBatch batch;
     for (int32_t s : fin) {
         Request& q = e->reqs[e->slot_req[s]];
         q.out.resize((size_t)6 * q.n);
+        const int64_t doubles = 6 * q.n;
+        if (doubles <= kStageDoubles && have_stage(e)) {
+            if (!batch.fits(doubles)) {
+                rc = flush_retirements(e, batch);
+                if (rc) return rc;
+            }
+            batch.add(&q, q.aoff, s, doubles);
+            continue;
+        }
         const size_t d = sizeof(double) * (size_t)q.n;
         const double* src[6] = {e->x, e->y, e->z, e->vx, e->vy, e->vz};
         for (int k = 0; k < 6; ++k)
@@ -529,6 +654,11 @@ int retire(nb_engine* e) {
                                   cudaMemcpyDeviceToHost, e->stream));
         NE_CK(nb::launch_fill_i32(e->sysid + q.aoff, q.n, -1, e->stream));
         NE_CK(cudaStreamSynchronize(e->stream));
+    }
+    rc = flush_retirements(e, batch);
+    if (rc) return rc;
+    for (int32_t s : fin) {
+        Request& q = e->reqs[e->slot_req[s]];
         free_range(e, q.aoff, q.n);
         q.state = NB_REQ_DONE;
         e->slot_req[s] = -1;
@@ -742,6 +872,8 @@ int nb_engine_destroy(nb_engine* e) {
     if (e->ev0) cudaEventDestroy(e->ev0);
     if (e->ev1) cudaEventDestroy(e->ev1);
     if (e->partial) cudaFree(e->partial);
+    if (e->stage) cudaFree(e->stage);
+    if (e->hstage) cudaFreeHost(e->hstage);
     cudaFree(e->arena);
     cudaStreamDestroy(e->stream);
     delete e;

@@ -302,6 +302,26 @@ struct BatchForce {
     const int64_t* nsteps_slot;
 };
 
+// One system of a batched admission or retirement: n particles at arena index
+// aoff, at src doubles in the staging buffer.
+struct BatchMove {
+    int64_t src;
+    int64_t aoff;
+    int32_t n;
+    int32_t slot;
+};
+struct BatchArrays {
+    double *x, *y, *z, *vx, *vy, *vz, *m, *ax, *ay, *az;
+    int32_t* sysid;
+    int64_t* steps_slot;
+};
+// Admission: x, y, z, vx, vy, vz, m (n each) from the staging buffer into the
+// arena, zero accelerations, the slot on every particle and no steps made.
+// Retirement: x, y, z, vx, vy, vz into the staging buffer, the particles free.
+cudaError_t launch_batch_admit(const BatchMove* moves, int32_t count, int32_t max_n, const double* stage,
+                               BatchArrays a, cudaStream_t s);
+cudaError_t launch_batch_retire(const BatchMove* moves, int32_t count, int32_t max_n, double* stage,
+                                BatchArrays a, cudaStream_t s);
 cudaError_t launch_force_batch(int law, const BatchForce& f, int grid, int block, int ipt,
                                cudaStream_t s);
 cudaError_t launch_fill_i32(int32_t* a, int64_t n, int32_t v, cudaStream_t s);
