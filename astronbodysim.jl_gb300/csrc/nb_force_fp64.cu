@@ -2,7 +2,8 @@
 //
 // Built with -fmad=false so every a*b+c rounds twice, as Julia evaluates the
 // pair expressions of src/directsum/gravity.jl:8-28 and
-// src/directsum/potential.jl:2-27; sqrt and division are IEEE-rounded.  Each
+// src/directsum/potential.jl:2-27; roots and quotients round as IEEE ones (see
+// root64 for the exceptions).  Each
 // pair term is therefore the same double the CPU computes; the per-target sum
 // is compensated (TwoSum), so the result differs from the CPU's pairwise sum
 // (src/directsum/gravity.jl:45) only by that sum's own rounding.
@@ -10,13 +11,16 @@
 // Sources are staged through shared memory in tiles of kTile (x, y, z, m);
 // one target per thread.
 //
-// What bounds it: the FP64 pipe (2 lanes per clock and SM on this GPU), about
-// 60 FP64-pipe operations per pair, so the time is pairs / (busy SMs).  One
+// What bounds it: the FP64 pipe (2 lanes per clock and SM on this GPU), so the
+// time is FP64 operations / busy SMs.  A pair took about 60 with the compiler's
+// square root and division and TwoSum for the three sums; it takes 37 with G = 1 (40 otherwise) with one
+// reciprocal root for both (root64, quotient64) and sums ordered on the integer
+// pipe (ordered_sum_acc): 9.6 -> 13.4 G interactions/s on a full GPU, the same
+// terms to the last bit in every case measured.  One
 // block of targets per CTA leaves most SMs idle below 152 x 8 blocks (N =
-// 4096: 32 CTAs on 152 SMs, 8.0 ms a force), so each block's sources are
+// 4096: 32 CTAs on 152 SMs, 8.0 ms a force at the former rate), so each block's sources are
 // split over js CTAs (fp64_split) whose compensated partial sums are joined
-// in part order by k_force_fp64_join: 1.76 ms a step at N = 4096, the rate
-// of a full GPU (9.6 G interactions/s).
+// in part order by k_force_fp64_join: 1.25 ms a step at N = 4096.
 #include "nb_internal.cuh"
 
 namespace nb {
@@ -40,61 +44,90 @@ __host__ __device__ __forceinline__ int fp64_split(int64_t nblocks, int64_t nsrc
 
 size_t fp64_partial_bytes() { return sizeof(double) * 8 * (size_t)kFp64Items * kTile; }
 
-template <int LAW>
-__device__ __forceinline__ void pair_force64(double px, double py, double pz, dvec4 q, double G,
-                                             double h, double h_inv, double h3_inv, double& fx,
-                                             double& fy, double& fz) {
-    const double dx = q.x - px, dy = q.y - py, dz = q.z - pz;
-    const double r2 = dx * dx + dy * dy + dz * dz;
-    double fac;
-    if (LAW == NB_LAW_PLUMMER) {
-        const double r2e = r2 + h * h;
-        fac = q.w / (r2e * sqrt(r2e));
-    } else {
-        const double r = sqrt(r2);
-        if (r >= h) {
-            fac = q.w / (r2 * r);
-        } else {
-            const double u = r * h_inv;
-            if (u < 0.5)
-                fac = q.w * h3_inv * (10.666666666667 + u * u * (32.0 * u - 38.4));
-            else
-                fac = q.w * h3_inv *
-                      (21.333333333333 - 48.0 * u + 38.4 * (u * u) - 10.666666666667 * (u * u * u) -
-                       0.066666666667 / (u * u * u));
-        }
-    }
-    fx = dx * fac * G;
-    fy = dy * fac * G;
-    fz = dz * fac * G;
+// (s, c) += v as two_sum_acc, with the operands ordered by exponent on the
+// integer pipe so that three additions give the rounding error (Dekker 1971)
+// instead of five; the same error, being exact either way.
+__device__ __forceinline__ void ordered_sum_acc(double& s, double& c, double v) {
+    const bool swap = (__double2hiint(v) & 0x7fffffff) > (__double2hiint(s) & 0x7fffffff);
+    const double a = swap ? v : s, b = swap ? s : v;
+    const double t = __dadd_rn(a, b);
+    c = __dadd_rn(c, __dadd_rn(b, -__dadd_rn(t, -a)));
+    s = t;
 }
 
-template <int LAW>
-__device__ __forceinline__ double pair_pot64(double px, double py, double pz, dvec4 q, double G,
-                                             double h, double h_inv) {
-    const double dx = q.x - px, dy = q.y - py, dz = q.z - pz;
-    const double r2 = dx * dx + dy * dy + dz * dz;
-    const double r = sqrt(r2);
-    double pot;
-    if (LAW == NB_LAW_PLUMMER) {
-        pot = -q.w / sqrt(r2 + h * h) * G;
-    } else if (r >= h) {
-        pot = -q.w / r * G;
-    } else {
-        const double u = r * h_inv;
-        double wp;
-        if (u < 0.5)
-            wp = -2.8 + u * u * (5.333333333333 + u * u * (6.4 * u - 9.6));
-        else
-            wp = -3.2 + 0.066666666667 / u +
-                 u * u * (10.666666666667 + u * (-16.0 + u * (9.6 - 2.133333333333 * u)));
-        pot = q.w * h_inv * wp * G;
-    }
-    if (r == 0.0) pot = pot * 0.0;
-    return pot;
+// r = sqrt(x) and y ~ 1 / sqrt(x).  From the hardware's approximation y0 one
+// step of Halley's iteration, y = y0 (1 + e/2 + 3 e^2 / 8) with e = 1 - x y0^2,
+// then r = x y corrected by its residual (Markstein 1990), which rounds like
+// an exact square root but for cases within a 2^-50th of a tie.  8 FP64-pipe
+// operations and a square root's reciprocal for the quotients below, which
+// then need no division of their own.  x within 2^-300 .. 2^300 (in_range).
+__device__ __forceinline__ bool in_range(double x) {
+    return (uint32_t)(__double2hiint(x) - ((1023 - 300) << 20)) < (uint32_t)(600 << 20);
+}
+__device__ __forceinline__ void root64(double x, double& r, double& y) {
+    double y0;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(x));
+    const double e = __fma_rn(-__dmul_rn(x, y0), y0, 1.0);
+    y = __fma_rn(__dmul_rn(y0, e), __fma_rn(0.375, e, 0.5), y0);
+    const double g = __dmul_rn(x, y);
+    // y / 2 by its exponent
+    const double hy = __hiloint2double(__double2hiint(y) - (1 << 20), __double2loint(y));
+    r = __fma_rn(__fma_rn(-g, g, x), hy, g);
+}
+// m / d, z ~ 1 / d within a few ulp: the product corrected by its residual.
+__device__ __forceinline__ double quotient64(double m, double d, double z) {
+    const double q = __dmul_rn(m, z);
+    return __fma_rn(__fma_rn(-q, d, m), z, q);
 }
 
+// Pair at separation (dx, dy, dz): acceleration factor fac (times the
+// separation and G) and potential pot (with G).
 template <int LAW, bool ACC, bool POT>
+__device__ __forceinline__ void pair64(double dx, double dy, double dz, double m, double G, double h,
+                                       double h_inv, double h3_inv, double& fac, double& pot) {
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    const double x = LAW == NB_LAW_PLUMMER ? r2 + h * h : r2;
+    double r, y;
+    const bool fast = in_range(x);
+    if (fast) {
+        root64(x, r, y);
+    } else {
+        r = sqrt(x);
+        y = 0.0;
+    }
+    // r >= h on the bit patterns: both are non-negative
+    if (LAW == NB_LAW_PLUMMER || __double_as_longlong(r) >= __double_as_longlong(h)) {
+        if (fast) {
+            if (ACC) fac = quotient64(m, x * r, __dmul_rn(__dmul_rn(y, y), y));
+            if (POT) pot = -quotient64(m, r, y) * G;
+        } else {
+            if (ACC) fac = m / (x * r);
+            if (POT) pot = -m / r * G;
+        }
+        if (LAW == NB_LAW_PLUMMER && POT && r2 == 0.0) pot = pot * 0.0;
+        return;
+    }
+    const double u = r * h_inv;
+    if (u < 0.5) {
+        if (ACC) fac = m * h3_inv * (10.666666666667 + u * u * (32.0 * u - 38.4));
+        if (POT) pot = m * h_inv * (-2.8 + u * u * (5.333333333333 + u * u * (6.4 * u - 9.6))) * G;
+        if (POT && r == 0.0) pot = pot * 0.0;
+    } else {
+        if (ACC)
+            fac = m * h3_inv *
+                  (21.333333333333 - 48.0 * u + 38.4 * (u * u) - 10.666666666667 * (u * u * u) -
+                   0.066666666667 / (u * u * u));
+        if (POT)
+            pot = m * h_inv *
+                  (-3.2 + 0.066666666667 / u +
+                   u * u * (10.666666666667 + u * (-16.0 + u * (9.6 - 2.133333333333 * u)))) *
+                  G;
+    }
+}
+
+// UNIT_G: G is exactly 1 (the default unit system), so the three products by it,
+// which change no bit, are left out.
+template <int LAW, bool ACC, bool POT, bool UNIT_G>
 __global__ void __launch_bounds__(kTile)
     k_force_fp64(Sources64 src, Targets tg, double G, double* __restrict__ partial) {
     __shared__ dvec4 sj[kTile];
@@ -127,14 +160,15 @@ __global__ void __launch_bounds__(kTile)
         const int cnt = (int)((jhi - j0) < kTile ? (jhi - j0) : kTile);
         for (int j = 0; j < cnt; ++j) {
             const dvec4 q = sj[j];
+            const double dx = q.x - px, dy = q.y - py, dz = q.z - pz;
+            double fac = 0.0, pot = 0.0;
+            pair64<LAW, ACC, POT>(dx, dy, dz, q.w, G, h, h_inv, h3_inv, fac, pot);
             if (ACC) {
-                double fx, fy, fz;
-                pair_force64<LAW>(px, py, pz, q, G, h, h_inv, h3_inv, fx, fy, fz);
-                two_sum_acc(sx, cx, fx);
-                two_sum_acc(sy, cy, fy);
-                two_sum_acc(sz, cz, fz);
+                ordered_sum_acc(sx, cx, UNIT_G ? dx * fac : dx * fac * G);
+                ordered_sum_acc(sy, cy, UNIT_G ? dy * fac : dy * fac * G);
+                ordered_sum_acc(sz, cz, UNIT_G ? dz * fac : dz * fac * G);
             }
-            if (POT) two_sum_acc(sp, cp, pair_pot64<LAW>(px, py, pz, q, G, h, h_inv));
+            if (POT) ordered_sum_acc(sp, cp, pot);
         }
     }
     if (js > 1) {
@@ -202,12 +236,17 @@ static cudaError_t launch_law(bool acc, bool pot, const Sources64& src, const Ta
     const bool split = js > 1 || (tg.d_count && fp64_split(1, src.n) > 1);
     int64_t grid = nblocks * js;
     if (tg.d_count && split && grid < kFp64Items) grid = kFp64Items;
+    const bool unit = G == 1.0;
+#define NB_FP64(A, P)                                                                             \
+    (unit ? k_force_fp64<LAW, A, P, true><<<(unsigned)grid, kTile, 0, s>>>(src, tg, G, partial)    \
+          : k_force_fp64<LAW, A, P, false><<<(unsigned)grid, kTile, 0, s>>>(src, tg, G, partial))
     if (acc && pot)
-        k_force_fp64<LAW, true, true><<<(unsigned)grid, kTile, 0, s>>>(src, tg, G, partial);
+        NB_FP64(true, true);
     else if (acc)
-        k_force_fp64<LAW, true, false><<<(unsigned)grid, kTile, 0, s>>>(src, tg, G, partial);
+        NB_FP64(true, false);
     else if (pot)
-        k_force_fp64<LAW, false, true><<<(unsigned)grid, kTile, 0, s>>>(src, tg, G, partial);
+        NB_FP64(false, true);
+#undef NB_FP64
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || !split) return e;
     // blocks that can be split: at most kFp64Items / 2

@@ -34,6 +34,22 @@ def test_fp64_split_matches_oracle(nb, oracle, n, law):
     assert np.abs((pot - p) / p).max() <= BAR
 
 
+@pytest.mark.parametrize("law", ["spline", "plummer"])
+@pytest.mark.parametrize("scale", [1e-60, 1e-46, 1e-3, 1e44, 1e46, 1e60])
+def test_fp64_roots_over_the_exponent_range(nb, oracle, scale, law):
+    """Lengths from 1e-60 to 1e60: squares inside, at the edges of and outside
+    the range of the fast root, where the compiler's takes over."""
+    n, h = 400, 0.02 * scale
+    d = nb.plummer(n, seed=8)
+    d["pos"] = d["pos"] * scale
+    sim = nb.Simulation(d, G=3.7, ForceSofteningTable=[h] * 6, TimeStep=1e-3, precision="fp64", law=law)
+    nb.compute_force(sim, want_potential=True)
+    g = nb.get_all_data(sim)
+    a, p = oracle.force(d["pos"], d["mass"], d["pos"], h, G=3.7, law=0 if law == "spline" else 1)
+    assert (np.abs(g["acc"] - a).max(1) / np.abs(a).max(1)).max() <= BAR
+    assert np.abs((g["pot"] - p) / p).max() <= BAR
+
+
 @pytest.mark.parametrize("n_active", [1, 128, 129, 2500])
 def test_fp64_split_with_active_list(nb, oracle, n_active):
     n, h = 3000, 0.02
