@@ -22,6 +22,8 @@
 // Potential (src/directsum/potential.jl:2-27): -m/r, spline inside h, 0 at r=0.
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include "nb_pairs.cuh"
 
 namespace nb {
@@ -223,6 +225,74 @@ struct ForceOcc {
         (BLOCK == 128 && !POT) ? (IPT == 1 ? NB_MINB_IPT1 : (IPT == 2 ? NB_MINB_IPT2 : NB_MINB_IPT4)) : 1;
 };
 
+// The clock update of a constant step whose drift ran in the pack (one thread).
+__device__ __forceinline__ void end_constant_step(const Targets& tg) {
+    Clock* c = tg.step_clk;
+    const double t = c->t_float;
+    c->t_float = __dadd_rn(t, tg.kick_dt);
+    c->dt_drift = __dadd_rn(c->t_float, -t);
+    c->last_t_float = c->t_float;  // src/run.jl:164
+    c->interactions = __dadd_rn(c->interactions, __dmul_rn((double)tg.n, (double)tg.n));
+    c->steps += 1;
+}
+
+// Join of a block whose parts are one cluster: every CTA leaves its compensated
+// sums in its shared memory (sum: 6 x kPer floats) and joins a js-th of the
+// block's targets from all of them, one (target, component) per thread, in part
+// order.  Against the join by the last CTA through global memory this saves
+// the sums' round trip through the L2, the count, and most of the time of the
+// FP64 epilogue, which one CTA's threads otherwise share the FP64 pipe of one
+// SM for: 5.7 of 19.5 us of a force launch at N = 4096, 3.7 of 7.4 at N = 1000.
+template <int BLOCK, int IPT>
+__device__ __forceinline__ void cluster_join(float* sum, int js, int part, int64_t base, int64_t ntg,
+                                             const float* sx, const float* cx, const float* sy,
+                                             const float* cy, const float* sz, const float* cz,
+                                             const Targets& tg, double G) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    constexpr int kPer = BLOCK * IPT;
+    const int tid = threadIdx.x;
+    __syncthreads();  // every warp is done with the tiles that sum overwrites
+#pragma unroll
+    for (int k = 0; k < IPT; ++k) {
+        float* q = sum + k * BLOCK + tid;
+        q[0 * kPer] = sx[k];
+        q[1 * kPer] = cx[k];
+        q[2 * kPer] = sy[k];
+        q[3 * kPer] = cy[k];
+        q[4 * kPer] = sz[k];
+        q[5 * kPer] = cz[k];
+    }
+    const int seg = (kPer + js - 1) / js, lo = part * seg;
+    cluster.sync();
+    for (int i = tid; i < 3 * seg; i += BLOCK) {
+        const int comp = i / seg, slot = lo + i % seg;
+        const int64_t t = base + slot;
+        if (slot >= kPer || t >= ntg) continue;
+        const int32_t p = tg.idx ? tg.idx[t] : (int32_t)t;
+        double* a = comp == 0 ? tg.ax : comp == 1 ? tg.ay : tg.az;
+        double* v = comp == 0 ? tg.vx : comp == 1 ? tg.vy : tg.vz;
+        const double vp = v ? v[p] : 0.0;
+        float s = 0.0f, c = 0.0f;
+#pragma unroll 8
+        for (int u = 0; u < js; ++u) {
+            const float* q = cluster.map_shared_rank(sum + 2 * comp * kPer + slot, u);
+            two_sum_acc(s, c, q[0]);
+            c += q[kPer];
+        }
+        const double acc = ((double)s + (double)c) * G;
+        a[p] = acc;
+        if (v) v[p] = __dadd_rn(vp, __dmul_rn(acc, tg.kick_dt));  // k_kick with constant steps
+    }
+    if (tg.step_clk && base == 0 && part == 0 && tid == 0) end_constant_step(tg);
+    cluster.sync();  // the last read of another CTA's shared memory
+}
+
+// The shape that small systems run in.  The others do without: its mere
+// presence changed the pair loop's schedule (N = 2^20: 344 -> 356 ms a step).
+template <int BLOCK, int IPT, int TJ, bool ACC, bool POT>
+constexpr bool kClusterJoin = BLOCK == 128 && IPT == 1 && TJ == 128 && ACC && !POT;
+
 template <int LAW, bool ACC, bool POT, int BLOCK, int IPT, int TJ, int NST>
 __global__ void __launch_bounds__(BLOCK, (ForceOcc<BLOCK, IPT, POT>::value)) k_force_mixed(Sources32 src, Targets tg, double G,
                                                        uint32_t* __restrict__ err) {
@@ -380,9 +450,17 @@ __global__ void __launch_bounds__(BLOCK, (ForceOcc<BLOCK, IPT, POT>::value)) k_f
                 (void)mbar_wait_bounded(&full[u % NST], (uint32_t)(u / NST) & 1u,
                                         kWaitTimeoutNs / 8);
         }
-        return;
+        // (a cluster's CTAs stay: the others read their shared memory)
+        if (!(kClusterJoin<BLOCK, IPT, TJ, ACC, POT> && src.cluster)) return;
     }
 
+    if constexpr (kClusterJoin<BLOCK, IPT, TJ, ACC, POT>) {
+        if (src.cluster) {
+            cluster_join<BLOCK, IPT>(reinterpret_cast<float*>(buf), js, part, base, ntg, sx, cx, sy, cy, sz,
+                                     cz, tg, G);
+            return;
+        }
+    }
     if (js > 1) {
         // Compensated partials of this CTA's tile range; the CTA that finishes
         // last adds its block's parts in part order as double-float numbers in
@@ -450,16 +528,7 @@ __global__ void __launch_bounds__(BLOCK, (ForceOcc<BLOCK, IPT, POT>::value)) k_f
             }
         }
     }
-    if (tg.step_clk && blk == 0 && tid == 0) {
-        // the clock update of a constant step whose drift ran in the pack
-        Clock* c = tg.step_clk;
-        const double t = c->t_float;
-        c->t_float = __dadd_rn(t, tg.kick_dt);
-        c->dt_drift = __dadd_rn(c->t_float, -t);
-        c->last_t_float = c->t_float;  // src/run.jl:164
-        c->interactions = __dadd_rn(c->interactions, __dmul_rn((double)tg.n, (double)tg.n));
-        c->steps += 1;
-    }
+    if (tg.step_clk && blk == 0 && tid == 0) end_constant_step(tg);
 #pragma unroll
     for (int k = 0; k < IPT; ++k) {
         if (pidx[k] < 0) continue;
@@ -490,6 +559,17 @@ __global__ void __launch_bounds__(BLOCK, (ForceOcc<BLOCK, IPT, POT>::value)) k_f
     }
 }
 
+// Small systems: the parts of each block as one cluster of up to 8 CTAs, the
+// portable size, while the clusters of all blocks run at once.  us a step with /
+// without clusters: N = 1000 14.5 / 16.6, 2048 16.5 / 18.6, 4096 22.7 / 25.4,
+// 8192 47.7 / 47.1, 16384 140 / 127.
+constexpr int kClusterParts = 8;
+constexpr int64_t kClusterBlocks = 48;
+inline bool cluster_split(const Sources32& src, const Targets& tg, int64_t nblk) {
+    return src.partial && src.jsplit == 0 && !tg.d_count && tg.split && src.ntiles > 1 &&
+           nblk <= kClusterBlocks;
+}
+
 // Launch of one force evaluation with tiles of TJ sources (instantiated in
 // nb_force_mixed_t<TJ>.cu).  Shapes: (128 | 256 threads) x (1 | 2 | 4 targets
 // per thread) with the default 4-stage ring; the acceleration-only form of
@@ -505,6 +585,25 @@ cudaError_t launch_cfg_tile(const Sources32& src, const Targets& tg, double G, u
     // kSplitItems items where that is more than 8 per block
     const int js = !src.partial ? 1 : src.jsplit > 0 ? src.jsplit : split_parts(nblk, src.ntiles);
     int64_t grid = nblk * js;
+    if constexpr (kClusterJoin<128, 1, TJ, ACC, POT>) {
+        if (block == 128 && ipt == 1 && stages == 4 && cluster_split(src, tg, nblk)) {
+            Sources32 sc = src;
+            sc.cluster = 1;
+            sc.jsplit = src.ntiles < kClusterParts ? src.ntiles : kClusterParts;
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3((unsigned)(nblk * sc.jsplit));
+            cfg.blockDim = dim3(128);
+            cfg.stream = s;
+            cudaLaunchAttribute at{};
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = (unsigned)sc.jsplit;
+            at.val.clusterDim.y = 1;
+            at.val.clusterDim.z = 1;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            return cudaLaunchKernelEx(&cfg, k_force_mixed<LAW, ACC, POT, 128, 1, TJ, 4>, sc, tg, G, err);
+        }
+    }
     if (src.partial && src.jsplit == 0 && tg.d_count) {
         const int64_t most = nblk * src.ntiles < kSplitItems ? nblk * src.ntiles : kSplitItems;
         if (grid < most) grid = most;

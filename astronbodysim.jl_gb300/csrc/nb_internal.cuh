@@ -167,7 +167,7 @@ struct Sources32 {
     // leaves it to split_parts() on the device's target count.  partial
     // nullptr: no split.
     int32_t jsplit;
-    int32_t pad;
+    int32_t cluster;  // the parts of a block are one cluster and join through its shared memory
     float* partial;
     uint32_t* done;
 };
