@@ -100,3 +100,26 @@ def test_active_list_is_split_on_the_device(nb, n_active):
     assert np.all(got[rest] == 7.0)
     e = np.linalg.norm(got[act] - ref[act], axis=1) / np.linalg.norm(ref[act], axis=1)
     assert np.median(e) <= 1e-6 and np.quantile(e, 0.99) <= 1e-5 and e.max() <= 1e-4
+
+
+@pytest.mark.parametrize("resort", [1, 3, 5, 16])
+@pytest.mark.parametrize("adaptive", [False, True])
+def test_steps_do_not_depend_on_how_they_are_asked_for(nb, resort, adaptive):
+    """Calls of 1 .. 17 steps replay graphs of one or four steps between the sorts:
+    the same states as one step at a time, bit for bit."""
+    d = nb.plummer(700, seed=2)
+    kw = dict(ForceSofteningTable=[0.02] * 6, TimeEnd=4.0, resort_every=resort, MaxStep=1e-2)
+    kw.update({} if adaptive else {"TimeStep": 1e-3})
+    a, b = nb.Simulation(d, **kw), nb.Simulation(d, **kw)
+    for s in (a, b):
+        nb.compute_force(s)
+        nb.init_timesteps(s)
+        nb.leapfrog_half_kick(s, +1)
+    for k in (1, 2, 9, 4, 17, 3, 5):
+        nb.step(a, k)
+        for _ in range(k):
+            nb.step(b, 1)
+        ga, gb = nb.get_all_data(a), nb.get_all_data(b)
+        for key in ("pos", "vel", "acc", "ti_endstep"):
+            np.testing.assert_array_equal(ga[key], gb[key])
+    assert a.time() == b.time() and nb.counters(a) == nb.counters(b)
