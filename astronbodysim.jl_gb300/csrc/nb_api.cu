@@ -43,13 +43,16 @@ struct nb_handle {
     int64_t diag_blocks = 0;
     double* diag_out = nullptr;
     Clock* clk = nullptr;
+    uint32_t* herr = nullptr;  // pinned copy of the clock's error word
     void* probe = nullptr;
     size_t probe_bytes = 0;
-    // Step graphs: [0] re-orders the sources (Morton sort) before the pack,
-    // [1] packs in the order of the last sort.  The host replays [0] every
-    // resort steps (and whenever the order is not valid) and [1] otherwise.
+    // Step graphs, captured when first needed: step_exec re-orders the sources
+    // (Morton sort) before the pack, the others pack in the order of the last
+    // sort, one step or kManySteps at a time.  The host replays the first every
+    // resort steps (and whenever the order is not valid).
     cudaGraphExec_t step_exec = nullptr;
     cudaGraphExec_t step_exec_nosort = nullptr;
+    cudaGraphExec_t step_exec_many = nullptr;  // kManySteps steps without the sort
     cudaGraphExec_t out_exec = nullptr;  // step graph that stops at output times
     cudaGraphExec_t out_exec_nosort = nullptr;
     int resort = 16;                      // steps between Morton sorts in the step graphs
@@ -98,6 +101,9 @@ constexpr int kAutoJsplitMax = 8;
 // two, 11.9 by four, 11.1 by eight; N = 4096: 22.9, 21.6, 20.7, 20.4), and the
 // 15 steps between two sorts are not a multiple of eight.
 constexpr int64_t kManySteps = 4;
+// Particles up to which nb_download joins evenly spaced arrays in one copy.
+constexpr int64_t kStridedCopyMax = 65536;
+constexpr ptrdiff_t kStridedCopyPitch = (ptrdiff_t)1 << 30;
 constexpr int64_t kAutoTile256From = 1 << 15;
 constexpr int64_t kAutoIpt2From = 1 << 16;
 constexpr int64_t kAutoTile512From = 1 << 17;
@@ -231,10 +237,12 @@ void drop_graph(nb_handle* h) {
     }
 }
 
+// Waits for the stream and reads the device's error word, which comes back with
+// the same wait (a copy of its own after it took 8 us).
 int sync_and_check(nb_handle* h) {
+    NB_CK(cudaMemcpyAsync(h->herr, &h->clk->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
     NB_CK(cudaStreamSynchronize(h->stream));
-    uint32_t e = 0;
-    NB_CK(cudaMemcpy(&e, &h->clk->err, sizeof e, cudaMemcpyDeviceToHost));
+    const uint32_t e = *h->herr;
     if (e) {
         NB_CK(cudaMemset(&h->clk->err, 0, sizeof e));
         if (e & nb::DEVERR_TIMEOUT)
@@ -754,7 +762,9 @@ int nb_create(const nb_params* p, nb_handle** out) {
     h->dev = p->device;
     if (cudaSetDevice(h->dev) != cudaSuccess ||
         cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMalloc(&h->clk, sizeof(Clock)) != cudaSuccess) {
+        cudaMalloc(&h->clk, sizeof(Clock)) != cudaSuccess ||
+        cudaHostAlloc(&h->herr, sizeof(uint32_t), cudaHostAllocDefault) != cudaSuccess) {
+        if (h->clk) cudaFree(h->clk);
         if (h->own_stream) cudaStreamDestroy(h->own_stream);
         delete h;
         return NB_ERR_CUDA;
@@ -790,6 +800,7 @@ int nb_create(const nb_params* p, nb_handle** out) {
         cudaMalloc(&h->sysdesc, sizeof(nb::SysDesc)) != cudaSuccess) {
         if (h->partial) cudaFree(h->partial);
         cudaFree(h->clk);
+        cudaFreeHost(h->herr);
         cudaStreamDestroy(h->own_stream);
         delete h;
         return NB_ERR_OOM;
@@ -806,6 +817,7 @@ int nb_destroy(nb_handle* h) {
     if (h->arena) cudaFree(h->arena);
     if (h->probe) cudaFree(h->probe);
     if (h->clk) cudaFree(h->clk);
+    if (h->herr) cudaFreeHost(h->herr);
     if (h->partial) cudaFree(h->partial);
     if (h->sysdesc) cudaFree(h->sysdesc);
     if (h->own_stream) cudaStreamDestroy(h->own_stream);
@@ -884,6 +896,11 @@ int nb_upload(nb_handle* h, int64_t n, const double* x, const double* y, const d
     return upload_sysdesc(h);
 }
 
+static bool pinned_host(const void* p) {
+    cudaPointerAttributes a{};
+    return cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type == cudaMemoryTypeHost;
+}
+
 int nb_download(nb_handle* h, double* x, double* y, double* z, double* vx, double* vy, double* vz,
                 double* ax, double* ay, double* az, double* pot, int64_t* ti_begstep,
                 int64_t* ti_endstep) {
@@ -893,17 +910,37 @@ int nb_download(nb_handle* h, double* x, double* y, double* z, double* vx, doubl
     if (h->n == 0) return NB_OK;
     const size_t d = sizeof(double) * (size_t)h->n;
     cudaStream_t s = h->stream;
-    struct {
-        void* dst;
-        const void* src;
-        size_t bytes;
-    } cp[] = {{x, h->x, d},   {y, h->y, d},   {z, h->z, d},   {vx, h->vx, d},
-              {vy, h->vy, d}, {vz, h->vz, d}, {ax, h->ax, d}, {ay, h->ay, d},
-              {az, h->az, d}, {pot, h->pot, d},
-              {ti_begstep, h->ti_beg, sizeof(int64_t) * (size_t)h->n},
-              {ti_endstep, h->ti_end, sizeof(int64_t) * (size_t)h->n}};
-    for (auto& c : cp)
-        if (c.dst) NB_CK(cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDeviceToHost, s));
+    double* const dst[10] = {x, y, z, vx, vy, vz, ax, ay, az, pot};
+    const double* const src[10] = {h->x,  h->y,  h->z,  h->vx, h->vy, h->vz,
+                                   h->ax, h->ay, h->az, h->pot};
+    // The arena's arrays are evenly spaced.  Runs of pinned host arrays that are
+    // so too go as one strided copy while the copies' own cost counts (ten steps
+    // of N = 1000 with the download of nine arrays: 221 -> 202 us).
+    const ptrdiff_t pitch = (const char*)h->y - (const char*)h->x;
+    for (int k = 0; k < 10;) {
+        int rows = 1;
+        if (dst[k] && h->n <= kStridedCopyMax) {
+            const ptrdiff_t step = k + 1 < 10 && dst[k + 1] ? (char*)dst[k + 1] - (char*)dst[k] : 0;
+            while (step >= (ptrdiff_t)d && step <= kStridedCopyPitch && k + rows < 10 && dst[k + rows] &&
+                   (char*)dst[k + rows] - (char*)dst[k + rows - 1] == step &&
+                   (const char*)src[k + rows] - (const char*)src[k + rows - 1] == pitch)
+                ++rows;
+            if (rows > 1 &&
+                !(pinned_host(dst[k]) && pinned_host(dst[k + rows - 1]) &&
+                  cudaMemcpy2DAsync(dst[k], (size_t)step, src[k], (size_t)pitch, d, (size_t)rows,
+                                    cudaMemcpyDeviceToHost, s) == cudaSuccess)) {
+                (void)cudaGetLastError();
+                rows = 1;
+            }
+        }
+        if (dst[k] && rows == 1) NB_CK(cudaMemcpyAsync(dst[k], src[k], d, cudaMemcpyDeviceToHost, s));
+        k += rows;
+    }
+    int64_t* const bins[2] = {ti_begstep, ti_endstep};
+    const int64_t* const bsrc[2] = {h->ti_beg, h->ti_end};
+    for (int k = 0; k < 2; ++k)
+        if (bins[k])
+            NB_CK(cudaMemcpyAsync(bins[k], bsrc[k], sizeof(int64_t) * (size_t)h->n, cudaMemcpyDeviceToHost, s));
     NB_CK(cudaStreamSynchronize(s));
     return NB_OK;
 }
