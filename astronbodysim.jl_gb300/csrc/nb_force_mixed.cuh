@@ -219,10 +219,16 @@ __global__ void __launch_bounds__(TJ) k_pack(const double* __restrict__ x,
 #ifndef NB_MINB_IPT4
 #define NB_MINB_IPT4 1
 #endif
-template <int BLOCK, int IPT, bool POT>
+// With the potential: alone 7 and 6 CTAs (one, two targets per thread; N = 50021:
+// 755 -> 720 us, N = 100003: 2483 -> 2402 us against the compiler's choice of 6
+// and 4), beside the acceleration 5 and its choice (1090 -> 1078 us).
+template <int BLOCK, int IPT, bool ACC, bool POT>
 struct ForceOcc {
     static constexpr int value =
-        (BLOCK == 128 && !POT) ? (IPT == 1 ? NB_MINB_IPT1 : (IPT == 2 ? NB_MINB_IPT2 : NB_MINB_IPT4)) : 1;
+        BLOCK != 128 ? 1
+        : !POT       ? (IPT == 1 ? NB_MINB_IPT1 : (IPT == 2 ? NB_MINB_IPT2 : NB_MINB_IPT4))
+        : ACC        ? (IPT == 1 ? 5 : 1)
+                     : (IPT == 1 ? 7 : (IPT == 2 ? 6 : 1));
 };
 
 // The clock update of a constant step whose drift ran in the pack (one thread).
@@ -294,7 +300,7 @@ template <int BLOCK, int IPT, int TJ, bool ACC, bool POT>
 constexpr bool kClusterJoin = BLOCK == 128 && IPT == 1 && TJ == 128 && ACC && !POT;
 
 template <int LAW, bool ACC, bool POT, int BLOCK, int IPT, int TJ, int NST>
-__global__ void __launch_bounds__(BLOCK, (ForceOcc<BLOCK, IPT, POT>::value)) k_force_mixed(Sources32 src, Targets tg, double G,
+__global__ void __launch_bounds__(BLOCK, (ForceOcc<BLOCK, IPT, ACC, POT>::value)) k_force_mixed(Sources32 src, Targets tg, double G,
                                                        uint32_t* __restrict__ err) {
     static_assert(TJ == 128 || TJ == 256 || TJ == 512, "tile of 128, 256 or 512 sources");
     constexpr int kWarpsPerCta = BLOCK / 32;
