@@ -290,14 +290,24 @@ bool fused_step(const nb_handle* h) {
            h->p.bg_kind == NB_BG_NONE && h->p.mond == NB_MOND_NONE;
 }
 
+// An adaptive step by the kernels of launch_adaptive_start: mixed precision on
+// the direct grid, with nothing between the force and the kick.  Five kernels
+// beside the force instead of ten.
+bool lean_adaptive_step(const nb_handle* h) {
+    return h->p.precision == NB_PREC_MIXED && h->p.adaptive && !h->worklist &&
+           h->p.bg_kind == NB_BG_NONE && h->p.mond == NB_MOND_NONE;
+}
+
 // Enqueue one force evaluation on stream s (no synchronisation).  With
 // active_only the targets are the particles with Ti_endstep == t_int
 // (src/directsum/gravity.jl:95-96); the list is built on the device.
 // sort = false packs the sources in the order of the last sort (perm must
 // hold a valid order; any order gives the same forces to FP32 round-off).
-// drift: the pack applies a constant step's drift first (fused_step only).
+// drift: the pack applies the step's drift first (fused_step and
+// lean_adaptive_step only); count: the pack counts the active particles for the
+// list (lean_adaptive_step only).
 cudaError_t enqueue_force(nb_handle* h, const nb::Targets& tg, cudaStream_t s, bool active_only,
-                          bool sort = true, bool drift = false) {
+                          bool sort = true, bool drift = false, bool count = false) {
     const bool pot = tg.pot != nullptr;
     const bool particles = tg.x == h->x;
     nb::Targets t2 = tg;
@@ -351,7 +361,12 @@ cudaError_t enqueue_force(nb_handle* h, const nb::Targets& tg, cudaStream_t s, b
         px.vy = h->vy;
         px.vz = h->vz;
         px.clk = h->clk;
-        px.dt = h->p.dt;
+        px.dt = h->p.adaptive ? 0.0 : h->p.dt;
+    }
+    if (count) {
+        px.clk = h->clk;
+        px.ti_end = h->ti_end;
+        px.counts = h->act_scratch;
     }
     e = nb::launch_pack(h->x, h->y, h->z, h->m, h->n, h->perm, h->tj, h->pack, h->origin, h->ext, px, s);
     if (e != cudaSuccess) return e;
@@ -397,7 +412,10 @@ cudaError_t enqueue_force(nb_handle* h, const nb::Targets& tg, cudaStream_t s, b
         // Targets are visited in the same Morton order, so the targets of a
         // warp are close together and most j-tiles take the branch-free loop.
         if (active_only) {
-            e = nb::launch_active_list(h->ti_end, h->n, h->perm, h->clk, h->active, h->act_scratch, s);
+            e = count ? nb::launch_active_from_counts(h->ti_end, h->n, h->perm, h->clk, h->active,
+                                                      h->act_scratch, s)
+                      : nb::launch_active_list(h->ti_end, h->n, h->perm, h->clk, h->active,
+                                               h->act_scratch, s);
             if (e != cudaSuccess) return e;
             t2.idx = h->active;
             t2.d_count = &h->clk->n_active;
@@ -456,6 +474,18 @@ cudaError_t enqueue_step(nb_handle* h, cudaStream_t s, bool sort) {
             if (e != cudaSuccess) return e;
         }
         return enqueue_force(h, t, s, false, sort, !sort);
+    }
+    if (lean_adaptive_step(h)) {
+        // the diagnostics' partials serve as the start's
+        e = nb::launch_adaptive_start(h->ti_end, h->n, h->tc, h->clk,
+                                      reinterpret_cast<int64_t*>(h->diag_scratch), s);
+        if (e == cudaSuccess && sort)  // the sort reads the drifted positions
+            e = nb::launch_drift_only(h->x, h->y, h->z, h->vx, h->vy, h->vz, h->n, h->clk, s);
+        if (e == cudaSuccess)
+            e = enqueue_force(h, particle_targets(h, true, false), s, true, sort, !sort, true);
+        if (e != cudaSuccess) return e;
+        return nb::launch_adaptive_kick(h->vx, h->vy, h->vz, h->ax, h->ay, h->az, h->type, h->ti_beg,
+                                        h->ti_end, h->n, h->tc, h->clk, h->active, s);
     }
     if (adaptive) {
         e = nb::launch_min_endstep(h->ti_end, h->n, h->p.time_base, h->clk, s);

@@ -36,9 +36,10 @@ namespace nb {
 // origin is the centre of the tile's FP64 bounding box, origin.w its half
 // diagonal.
 // ---------------------------------------------------------------------------
-// Optional extras (PackExtra): with DRIFT each particle takes its constant-step
-// drift first, in the operation order of k_drift (the step's own kernel for it
-// read and wrote the same positions once more); the split positions go out by
+// Optional extras (PackExtra): with DRIFT each particle takes its step's drift
+// first, in the operation order of k_drift (the step's own kernel for it read
+// and wrote the same positions once more); the active particles are counted for
+// the active list; the split positions go out by
 // slot for the force kernel, which otherwise gathers and splits them anew in
 // every CTA (12 FP64-pipe operations per target, 0.4 us of an SM's FP64 pipe
 // per 128 targets).
@@ -69,7 +70,8 @@ __global__ void __launch_bounds__(TJ) k_pack(const double* __restrict__ x,
     if (valid) {
         const int64_t p = perm ? (int64_t)perm[i] : i;
         if (DRIFT) {
-            const double t = e.clk->t_float, dt = __dadd_rn(__dadd_rn(t, e.dt), -t);
+            const double t = e.clk->t_float;
+            const double dt = e.dt > 0.0 ? __dadd_rn(__dadd_rn(t, e.dt), -t) : e.clk->dt_drift;
             px = __dadd_rn(e.x[p], __dmul_rn(e.vx[p], dt));
             py = __dadd_rn(e.y[p], __dmul_rn(e.vy[p], dt));
             pz = __dadd_rn(e.z[p], __dmul_rn(e.vz[p], dt));
@@ -83,6 +85,18 @@ __global__ void __launch_bounds__(TJ) k_pack(const double* __restrict__ x,
         }
         pm = m[p];
         if (e.split) hs = (float)(e.type ? e.soft[e.type[p] - 1] : e.h_const);
+    }
+    if (e.counts) {
+        // active particles (Ti_endstep == t_int) per 128 slots
+        __shared__ uint32_t wact[TJ / 32];
+        const bool act = valid && e.ti_end[perm ? (int64_t)perm[i] : i] == e.clk->t_int;
+        const unsigned mask = __ballot_sync(0xffffffffu, act);
+        if ((threadIdx.x & 31) == 0) wact[threadIdx.x >> 5] = __popc(mask);
+        __syncthreads();
+        if ((threadIdx.x & 127) == 0) {
+            const uint32_t* w = wact + (threadIdx.x >> 5);
+            if (i < n) e.counts[i >> 7] = w[0] + w[1] + w[2] + w[3];
+        }
     }
     const float2 sx = split_df(px), sy = split_df(py), sz = split_df(pz);
     if (e.split && valid) {

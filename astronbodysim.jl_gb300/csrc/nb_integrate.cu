@@ -144,23 +144,16 @@ cudaError_t launch_half_kick(double* vx, double* vy, double* vz, const double* a
     return cudaGetLastError();
 }
 
-// src/base/Timestep.jl:47-93 (advance_and_find_timestep)
-__global__ void k_kick(double* __restrict__ vx, double* __restrict__ vy, double* __restrict__ vz,
-                       const double* __restrict__ ax, const double* __restrict__ ay,
-                       const double* __restrict__ az, const int32_t* __restrict__ type,
-                       int64_t* __restrict__ ti_beg, int64_t* __restrict__ ti_end, int64_t n,
-                       TimeCfg c, Clock* clk) {
-    const int64_t i = (int64_t)blockIdx.x * kBlock + threadIdx.x;
-    if (i >= n) return;
-    if (!c.adaptive) {
-        vx[i] = vx[i] + ax[i] * c.dt;
-        vy[i] = vy[i] + ay[i] * c.dt;
-        vz[i] = vz[i] + az[i] * c.dt;
-        return;
-    }
-    const int64_t now = clk->t_int;
-    const int64_t te = ti_end[i];
-    if (te != now) return;
+// src/base/Timestep.jl:47-93 (advance_and_find_timestep) for a particle with
+// Ti_endstep == t_int.
+__device__ __forceinline__ void kick_active(double* __restrict__ vx, double* __restrict__ vy,
+                                            double* __restrict__ vz, const double* __restrict__ ax,
+                                            const double* __restrict__ ay,
+                                            const double* __restrict__ az,
+                                            const int32_t* __restrict__ type,
+                                            int64_t* __restrict__ ti_beg, int64_t* __restrict__ ti_end,
+                                            int64_t i, int64_t now, const TimeCfg& c, Clock* clk) {
+    const int64_t te = now;
     const int64_t TB = c.time_base;
     const double a_x = ax[i], a_y = ay[i], a_z = az[i];
     int64_t ti_step = get_timestep(a_x, a_y, a_z, c.soft[type[i] - 1], c, &clk->err);
@@ -176,6 +169,24 @@ __global__ void k_kick(double* __restrict__ vx, double* __restrict__ vy, double*
     ti_beg[i] = te;
     ti_end[i] = te + ti_step;
     if (!(isfinite(a_x) && isfinite(a_y) && isfinite(a_z))) atomicOr(&clk->err, DEVERR_NONFINITE);
+}
+
+__global__ void k_kick(double* __restrict__ vx, double* __restrict__ vy, double* __restrict__ vz,
+                       const double* __restrict__ ax, const double* __restrict__ ay,
+                       const double* __restrict__ az, const int32_t* __restrict__ type,
+                       int64_t* __restrict__ ti_beg, int64_t* __restrict__ ti_end, int64_t n,
+                       TimeCfg c, Clock* clk) {
+    const int64_t i = (int64_t)blockIdx.x * kBlock + threadIdx.x;
+    if (i >= n) return;
+    if (!c.adaptive) {
+        vx[i] = vx[i] + ax[i] * c.dt;
+        vy[i] = vy[i] + ay[i] * c.dt;
+        vz[i] = vz[i] + az[i] * c.dt;
+        return;
+    }
+    const int64_t now = clk->t_int;
+    if (ti_end[i] != now) return;
+    kick_active(vx, vy, vz, ax, ay, az, type, ti_beg, ti_end, i, now, c, clk);
 }
 
 cudaError_t launch_kick(double* vx, double* vy, double* vz, const double* ax, const double* ay,
@@ -305,6 +316,135 @@ cudaError_t launch_sync_count(const int64_t* ti_end, int64_t n, const Clock* clk
     return cudaGetLastError();
 }
 
+// ---------------------------------------------------------------------------
+// The adaptive step in five kernels beside the pack and the force's own: start
+// (min end step, clock), [pack: drift, counts], list, [force], kick (with the
+// clock's end of the step).  It took eleven (three for the start, three for the
+// list, drift, kick and clock of their own), of which a substep with few active
+// particles is mostly made: 12 substeps of 2 x 16384 particles 1205 -> 1096 us.
+// ---------------------------------------------------------------------------
+constexpr int64_t kStartBlocks = 1216;
+
+__global__ void __launch_bounds__(kBlock)
+    k_adaptive_start(const int64_t* __restrict__ ti_end, int64_t n, TimeCfg c, Clock* clk,
+                     int64_t* __restrict__ part) {
+    __shared__ long long red[kBlock / 32];
+    __shared__ int last;
+    long long v = LLONG_MAX;
+    for (int64_t i = (int64_t)blockIdx.x * kBlock + threadIdx.x; i < n; i += (int64_t)gridDim.x * kBlock)
+        v = min(v, (long long)ti_end[i]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kBlock / 32; ++w) v = min(v, red[w]);
+        __stcg((long long*)part + blockIdx.x, v);
+        __threadfence();  // the minimum before the ticket
+        last = atomicAdd(&clk->ticket, 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();  // the ticket before the others' minima
+    v = c.time_base;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += kBlock) v = min(v, __ldcg((const long long*)part + b));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kBlock / 32; ++w) v = min(v, red[w]);
+        clk->ticket = 0;
+        clk->min_endstep = v;
+        clk->last_t_int = clk->t_int;  // as k_clock_advance, mode 0
+        clk->t_int = v;
+        clk->t_float = c.time_begin + (double)clk->t_int * c.time_interval;
+        clk->dt_drift = (double)(clk->t_int - clk->last_t_int) * c.time_interval;
+    }
+}
+
+cudaError_t launch_adaptive_start(const int64_t* ti_end, int64_t n, TimeCfg cfg, Clock* clk,
+                                  int64_t* part, cudaStream_t s) {
+    int64_t g = (n + kBlock - 1) / kBlock;
+    if (g > kStartBlocks) g = kStartBlocks;
+    k_adaptive_start<<<(unsigned)g, kBlock, 0, s>>>(ti_end, n, cfg, clk, part);
+    return cudaGetLastError();
+}
+
+// Active list from the counts of every 128 slots.  SCANNED: counts hold the
+// exclusive sums; otherwise every block adds the counts before its own, which
+// for the sizes it is used for costs less than a scan kernel.
+template <bool SCANNED>
+__global__ void __launch_bounds__(kBlock)
+    k_active_list(const int64_t* __restrict__ ti_end, int64_t n, const int32_t* __restrict__ perm,
+                  Clock* clk, const uint32_t* __restrict__ counts, int32_t* __restrict__ list) {
+    static_assert(kBlock == 128, "counts of 128 slots");
+    __shared__ uint32_t wcount[kBlock / 32], wsum[kBlock / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t sum = 0;
+    if (!SCANNED) {
+        for (unsigned b = threadIdx.x; b < blockIdx.x; b += kBlock) sum += counts[b];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    }
+    int32_t i;
+    const bool act = slot_active(ti_end, n, perm, clk->t_int, (int64_t)blockIdx.x * kBlock + threadIdx.x, i);
+    const unsigned mask = __ballot_sync(0xffffffffu, act);
+    if (lane == 0) {
+        wcount[warp] = __popc(mask);
+        wsum[warp] = sum;
+    }
+    __syncthreads();
+    uint32_t base = SCANNED ? counts[blockIdx.x] : 0u, before = 0, total = 0;
+    for (int w = 0; w < kBlock / 32; ++w) {
+        if (!SCANNED) base += wsum[w];
+        if (w < warp) before += wcount[w];
+        total += wcount[w];
+    }
+    if (act) list[base + before + __popc(mask & ((1u << lane) - 1u))] = i;
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) clk->n_active = (int32_t)(base + total);
+}
+
+// Up to 131072 particles (1024 counts) every block sums for itself.
+cudaError_t launch_active_from_counts(const int64_t* ti_end, int64_t n, const int32_t* perm, Clock* clk,
+                                      int32_t* list, uint32_t* counts, cudaStream_t s) {
+    const unsigned g = grid_for(n);
+    if (g <= 1024) {
+        k_active_list<false><<<g, kBlock, 0, s>>>(ti_end, n, perm, clk, counts, list);
+        return cudaGetLastError();
+    }
+    cudaError_t e = launch_exclusive_scan(counts, (int64_t)g, s);
+    if (e != cudaSuccess) return e;
+    k_active_list<true><<<g, kBlock, 0, s>>>(ti_end, n, perm, clk, counts, list);
+    return cudaGetLastError();
+}
+
+// Kick of the listed particles, and the end of the step on the clock.
+__global__ void __launch_bounds__(kBlock)
+    k_adaptive_kick(double* __restrict__ vx, double* __restrict__ vy, double* __restrict__ vz,
+                    const double* __restrict__ ax, const double* __restrict__ ay,
+                    const double* __restrict__ az, const int32_t* __restrict__ type,
+                    int64_t* __restrict__ ti_beg, int64_t* __restrict__ ti_end, int64_t n, TimeCfg c,
+                    Clock* clk, const int32_t* __restrict__ list) {
+    const int64_t k = (int64_t)blockIdx.x * kBlock + threadIdx.x;
+    const int64_t count = clk->n_active;
+    if (k == 0) {  // as k_clock_end_step
+        clk->interactions += (double)count * (double)n;
+        clk->steps += 1;
+    }
+    if (k >= count) return;
+    kick_active(vx, vy, vz, ax, ay, az, type, ti_beg, ti_end, list[k], clk->t_int, c, clk);
+}
+
+cudaError_t launch_adaptive_kick(double* vx, double* vy, double* vz, const double* ax, const double* ay,
+                                 const double* az, const int32_t* type, int64_t* ti_beg, int64_t* ti_end,
+                                 int64_t n, TimeCfg cfg, Clock* clk, const int32_t* list, cudaStream_t s) {
+    if (n <= 0) return cudaSuccess;
+    k_adaptive_kick<<<grid_for(n), kBlock, 0, s>>>(vx, vy, vz, ax, ay, az, type, ti_beg, ti_end, n, cfg,
+                                                   clk, list);
+    return cudaGetLastError();
+}
+
 // Clock advance before a drift (single thread).
 //   mode 0: adaptive, to min_endstep       (src/directsum/timestep.jl:1-20)
 //   mode 1: adaptive, to t_int_arg
@@ -342,6 +482,12 @@ cudaError_t launch_drift(double* x, double* y, double* z, const double* vx, cons
                          const double* vz, int64_t n, TimeCfg cfg, Clock* clk, int mode,
                          int64_t t_int_arg, double t_float_arg, cudaStream_t s) {
     k_clock_advance<<<1, 1, 0, s>>>(clk, cfg, mode, t_int_arg, t_float_arg);
+    if (n > 0) k_drift<<<grid_for(n), kBlock, 0, s>>>(x, y, z, vx, vy, vz, n, clk);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_drift_only(double* x, double* y, double* z, const double* vx, const double* vy,
+                              const double* vz, int64_t n, const Clock* clk, cudaStream_t s) {
     if (n > 0) k_drift<<<grid_for(n), kBlock, 0, s>>>(x, y, z, vx, vy, vz, n, clk);
     return cudaGetLastError();
 }

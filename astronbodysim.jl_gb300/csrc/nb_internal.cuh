@@ -73,7 +73,7 @@ struct Clock {
     int32_t mid_step;         // 1: positions sit at an output time inside a step
     int32_t at_output;        // 1: stopped at an output, waiting for the host
     int32_t drift_skip;       // 1: the gated drift of this replay does nothing
-    int32_t pad;
+    int32_t ticket;           // finished blocks of k_adaptive_start, 0 between launches
     int64_t outputs;          // output stops so far
 };
 
@@ -130,9 +130,11 @@ struct Targets {
     Clock* step_clk;
 };
 
-// What the pack does beside packing, all optional: the constant-step drift of
-// each particle before it is packed (vx set: x += v * ((t + dt) - t), t read
-// from the clock, which the force's epilogue advances), the targets' split
+// What the pack does beside packing, all optional: the drift of each particle
+// before it is packed (vx set: with dt > 0 a constant step's, x += v * ((t +
+// dt) - t), t read from the clock, which the force's epilogue advances; with
+// dt = 0 by the clock's dt_drift), the number of active particles in every 128
+// slots (counts set, needs ti_end and the clock), the targets' split
 // positions (split[2 i], split[2 i + 1] = (x.hi, x.lo, y.hi, y.lo),
 // (z.hi, z.lo, h, 0) of slot i), and the zeroed join counters of the force.
 struct PackExtra {
@@ -150,6 +152,8 @@ struct PackExtra {
     double h_const;
     uint32_t* done;
     int32_t ndone;
+    const int64_t* ti_end;
+    uint32_t* counts;
 };
 
 // Packed FP32 sources for the mixed kernel: j-tiles of tile_j particles,
@@ -401,6 +405,20 @@ size_t fp64_partial_bytes();
 cudaError_t launch_active_list(const int64_t* ti_end, int64_t n, const int32_t* perm, Clock* clk,
                                int32_t* list, uint32_t* scratch, cudaStream_t s);
 int64_t active_scratch_words(int64_t n);
+// The adaptive step in few kernels.  Start: min_endstep and the clock's advance
+// to it (as launch_min_endstep and mode 0 of launch_drift, without the drift);
+// part: 8 bytes per 128 particles, at most 1216.  List: the active list from the
+// counts of the pack.  Kick: k_kick of the listed particles and the clock's end
+// of the step.
+cudaError_t launch_adaptive_start(const int64_t* ti_end, int64_t n, TimeCfg cfg, Clock* clk,
+                                  int64_t* part, cudaStream_t s);
+cudaError_t launch_active_from_counts(const int64_t* ti_end, int64_t n, const int32_t* perm, Clock* clk,
+                                      int32_t* list, uint32_t* counts, cudaStream_t s);
+cudaError_t launch_adaptive_kick(double* vx, double* vy, double* vz, const double* ax, const double* ay,
+                                 const double* az, const int32_t* type, int64_t* ti_beg, int64_t* ti_end,
+                                 int64_t n, TimeCfg cfg, Clock* clk, const int32_t* list, cudaStream_t s);
+cudaError_t launch_drift_only(double* x, double* y, double* z, const double* vx, const double* vy,
+                              const double* vz, int64_t n, const Clock* clk, cudaStream_t s);
 cudaError_t launch_exclusive_scan(uint32_t* counts, int64_t len, cudaStream_t s);
 cudaError_t launch_init_timesteps(const double* ax, const double* ay, const double* az,
                                   const int32_t* type, int64_t* ti_beg, int64_t* ti_end, int64_t n,

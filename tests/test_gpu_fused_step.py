@@ -123,3 +123,31 @@ def test_steps_do_not_depend_on_how_they_are_asked_for(nb, resort, adaptive):
         for key in ("pos", "vel", "acc", "ti_endstep"):
             np.testing.assert_array_equal(ga[key], gb[key])
     assert a.time() == b.time() and nb.counters(a) == nb.counters(b)
+
+
+@pytest.mark.parametrize("n", [1, 127, 129, 1000, 33000, 131072, 131073])
+def test_adaptive_step_is_the_step_of_single_operations(nb, n):
+    """Start, pack with drift and counts, list and kick of the adaptive step
+    against min end step, drift, force and kick as calls of their own: the same
+    operations, so bit-identical (the last sizes: lists from counts that each
+    block sums, and from a scan)."""
+    d = _data(nb, n)
+    d["collection"] = np.random.default_rng(n + 1).integers(1, 7, n)
+    kw = dict(ForceSofteningTable=[0.01, 0.02, 0.005, 0.03, 0.01, 0.04], TimeEnd=4.0, MaxStep=1e-2, resort_every=1)
+    a, b = nb.Simulation(d, **kw), nb.Simulation(d, **kw)
+    for s in (a, b):
+        nb.compute_force(s)
+        nb.init_timesteps(s)
+        nb.leapfrog_half_kick(s, +1)
+    total = 0.0
+    for _ in range(6):
+        nb.step(a, 1)
+        nb.drift_particles_adaptive_timestep(b, nb.find_min_endstep(b))
+        total += float(nb.active_count(b)) * n
+        nb.compute_force(b)
+        nb.advance_and_find_timestep(b)
+        ga, gb = nb.get_all_data(a), nb.get_all_data(b)
+        for k in ("pos", "vel", "acc", "ti_begstep", "ti_endstep"):
+            np.testing.assert_array_equal(ga[k], gb[k])
+        assert a.time() == b.time()
+    assert nb.counters(a) == (6, total)
