@@ -15,8 +15,8 @@
 // 125 us at N = 4096 and 200 us at N = 65536.  It runs instead as one cluster
 // of up to 16 CTAs whose shared memory holds all keys, passes separated by
 // hardware cluster barriers, digit counts and keys exchanged through
-// distributed shared memory (k_sort_cluster): 34 us at N = 4096, 107 us at
-// N = 65536, 173 us (277 as a chain) at N = 131072.  Larger sorts, bound by their
+// distributed shared memory (k_sort_cluster): 35 us at N = 4096, 86 us at
+// N = 65536, 143 us (277 as a chain) at N = 131072.  Larger sorts, bound by their
 // passes over memory, and GPUs without room for the cluster keep the chain:
 // per-block digit histograms -> one exclusive scan -> stable scatter that ranks
 // equal digits by (round, warp, lane) order.
@@ -344,46 +344,61 @@ cudaError_t launch_exclusive_scan(uint32_t* counts, int64_t len, cudaStream_t s)
 
 // ---------------------------------------------------------------------------
 // Radix sort in one cluster.  CTA c of C holds positions [c M, (c + 1) M) of
-// the current order, M = kCsThreads * ITEMS, in shared memory (keys and values,
+// the current order, M = THREADS * ITEMS, in shared memory (keys and values,
 // double-buffered).  A pass:
 //   * every warp ranks its 32 * ITEMS consecutive keys by digit, in order
-//     (match_any per round, running counts per warp and digit), and the CTA
+//     (votes per round, running counts per warp and digit), and the CTA
 //     turns the warps' counts into offsets and publishes its digit counts;
 //   * after a cluster barrier each CTA reads all CTAs' counts, which gives
 //     the first position of each of its digits in the whole order;
-//   * keys and values go to their positions in the other buffer of the CTA
-//     that owns them (distributed shared memory); cluster barrier.
+//   * keys and values are put in digit order within the CTA, so that a warp
+//     then writes a few runs and not 32 scattered words to their positions in
+//     the other buffers of the CTAs that own them (distributed shared memory);
+//     cluster barrier.
 // Stable, so the permutation is the same as that of the chain of kernels.
 // Positions past n are not stored; only the last CTAs have such.
 // ---------------------------------------------------------------------------
-constexpr int kCsThreads = 512;
-constexpr int kCsWarps = kCsThreads / 32;
-constexpr int kCsMaxItems = 16;
 constexpr int kCsMaxCluster = 16;
-constexpr int64_t kClusterSortMax = (int64_t)kCsMaxCluster * kCsThreads * kCsMaxItems;
+constexpr int64_t kClusterSortMax = (int64_t)kCsMaxCluster * 1024 * 8;
 
-template <int ITEMS>
+template <int THREADS, int ITEMS>
 struct CsShared {
-    uint64_t key[2][kCsThreads * ITEMS];
-    int32_t val[2][kCsThreads * ITEMS];
-    uint32_t cnt[kCsWarps][kRadix];  // per warp: counts, then offsets within the CTA
+    uint64_t key[2][THREADS * ITEMS];
+    int32_t val[2][THREADS * ITEMS];
+    uint16_t cnt[THREADS / 32][kRadix];  // per warp: counts, then offsets within the CTA (< 2^16)
     uint32_t total[kRadix];          // this CTA's digit counts, read by the others
     uint32_t base[kRadix];           // first position of each of its digits
-    uint32_t wsum[kRadix / 32];
+    uint32_t start[kRadix];          // first of each digit among this CTA's own keys in digit order
+    uint32_t wsum[2][kRadix / 32];
 };
 
-template <int ITEMS>
-__global__ void __launch_bounds__(kCsThreads)
+// The lanes with this lane's digit, among the valid ones.  A vote per bit beats
+// match_any here; with the runs above it took a sort of 65536 from 106 to 86 us,
+// of 131072 from 172 to 143 us, of 30000 from 69 to 61 us.
+__device__ __forceinline__ uint32_t same_digit(uint32_t d, bool valid) {
+    uint32_t peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+    for (int b = 0; b < kRadixBits; ++b) {
+        const bool bit = (d >> b) & 1u;
+        const uint32_t v = __ballot_sync(0xffffffffu, bit);
+        peers &= bit ? v : ~v;
+    }
+    return peers;
+}
+
+template <int THREADS, int ITEMS>
+__global__ void __launch_bounds__(THREADS)
     k_sort_cluster(const uint64_t* __restrict__ keys, int32_t* __restrict__ vals, int n, int passes) {
     namespace cg = cooperative_groups;
     extern __shared__ __align__(16) unsigned char cs_raw[];
-    CsShared<ITEMS>& sh = *reinterpret_cast<CsShared<ITEMS>*>(cs_raw);
+    using Shared = CsShared<THREADS, ITEMS>;
+    Shared& sh = *reinterpret_cast<Shared*>(cs_raw);
     cg::cluster_group cluster = cg::this_cluster();
-    constexpr int M = kCsThreads * ITEMS;
+    constexpr int M = THREADS * ITEMS, kWarpsOf = THREADS / 32;
     const int C = (int)cluster.num_blocks(), c = (int)cluster.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int first = c * M, count = min(M, max(0, n - first));  // keys this CTA holds
-    for (int i = tid; i < count; i += kCsThreads) {
+    for (int i = tid; i < count; i += THREADS) {
         sh.key[0][i] = keys[first + i];
         sh.val[0][i] = vals[first + i];
     }
@@ -394,34 +409,37 @@ __global__ void __launch_bounds__(kCsThreads)
         for (int d = lane; d < kRadix; d += 32) sh.cnt[warp][d] = 0;
         __syncwarp();
         uint64_t key[ITEMS];
+        int32_t val[ITEMS];
         uint32_t rank[ITEMS];
 #pragma unroll
         for (int r = 0; r < ITEMS; ++r) {
             const int i = warp * 32 * ITEMS + r * 32 + lane;
             const bool valid = i < count;
             key[r] = valid ? sh.key[src][i] : 0ull;
-            const uint32_t d = valid ? (uint32_t)(key[r] >> shift) & (kRadix - 1) : (uint32_t)kRadix;
-            const uint32_t peers = __match_any_sync(0xffffffffu, d);
+            val[r] = valid ? sh.val[src][i] : 0;
+            const uint32_t d = (uint32_t)(key[r] >> shift) & (kRadix - 1);
+            const uint32_t peers = same_digit(d, valid);
             const uint32_t before = __popc(peers & ((1u << lane) - 1u));
             rank[r] = valid ? sh.cnt[warp][d] + before : 0u;
             __syncwarp();
-            if (valid && before == 0u) sh.cnt[warp][d] += __popc(peers);
+            if (valid && before == 0u) sh.cnt[warp][d] += (uint16_t)__popc(peers);
             __syncwarp();
         }
         __syncthreads();
         if (tid < kRadix) {
             uint32_t run = 0;
 #pragma unroll
-            for (int w = 0; w < kCsWarps; ++w) {
+            for (int w = 0; w < kWarpsOf; ++w) {
                 const uint32_t v = sh.cnt[w][tid];
-                sh.cnt[w][tid] = run;
+                sh.cnt[w][tid] = (uint16_t)run;
                 run += v;
             }
             sh.total[tid] = run;
         }
         cluster.sync();
-        uint32_t all = 0, prev = 0, incl = 0;
+        uint32_t all = 0, prev = 0, own = 0, incl = 0, iown = 0;
         if (tid < kRadix) {
+            own = sh.total[tid];
 #pragma unroll 8
             for (int k = 0; k < C; ++k) {
                 const uint32_t v = *cluster.map_shared_rank(&sh.total[tid], k);
@@ -429,18 +447,30 @@ __global__ void __launch_bounds__(kCsThreads)
                 prev += k < c ? v : 0u;
             }
             incl = all;
+            iown = own;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += v;
+                const uint32_t u = __shfl_up_sync(0xffffffffu, iown, o);
+                if (lane >= o) {
+                    incl += v;
+                    iown += u;
+                }
             }
-            if (lane == 31) sh.wsum[warp] = incl;
+            if (lane == 31) {
+                sh.wsum[0][warp] = incl;
+                sh.wsum[1][warp] = iown;
+            }
         }
         __syncthreads();
         if (tid < kRadix) {
-            uint32_t b = incl - all + prev;
-            for (int w = 0; w < warp; ++w) b += sh.wsum[w];
+            uint32_t b = incl - all + prev, l = iown - own;
+            for (int w = 0; w < warp; ++w) {
+                b += sh.wsum[0][w];
+                l += sh.wsum[1][w];
+            }
             sh.base[tid] = b;
+            sh.start[tid] = l;
         }
         __syncthreads();
 #pragma unroll
@@ -448,35 +478,43 @@ __global__ void __launch_bounds__(kCsThreads)
             const int i = warp * 32 * ITEMS + r * 32 + lane;
             if (i < count) {
                 const uint32_t d = (uint32_t)(key[r] >> shift) & (kRadix - 1);
-                const uint32_t pos = sh.base[d] + sh.cnt[warp][d] + rank[r];
-                const int to = (int)(pos / M), at = (int)(pos % M);
-                *cluster.map_shared_rank(&sh.key[src ^ 1][at], to) = key[r];
-                *cluster.map_shared_rank(&sh.val[src ^ 1][at], to) = sh.val[src][i];
+                const uint32_t at = sh.start[d] + sh.cnt[warp][d] + rank[r];
+                sh.key[src][at] = key[r];
+                sh.val[src][at] = val[r];
             }
+        }
+        __syncthreads();
+        for (int i = tid; i < count; i += THREADS) {
+            const uint64_t k = sh.key[src][i];
+            const uint32_t d = (uint32_t)(k >> shift) & (kRadix - 1);
+            const uint32_t pos = sh.base[d] + ((uint32_t)i - sh.start[d]);
+            const int to = (int)(pos / M), at = (int)(pos % M);
+            *cluster.map_shared_rank(&sh.key[src ^ 1][at], to) = k;
+            *cluster.map_shared_rank(&sh.val[src ^ 1][at], to) = sh.val[src][i];
         }
         // all keys have arrived; also the last read of total, and of a CTA's
         // shared memory by another, before it is written again or given up
         cluster.sync();
     }
-    for (int i = tid; i < count; i += kCsThreads) vals[first + i] = sh.val[passes & 1][i];
+    for (int i = tid; i < count; i += THREADS) vals[first + i] = sh.val[passes & 1][i];
 }
 
-// Launches the cluster sort of n <= C * kCsThreads * ITEMS keys; *done false:
+// Launches the cluster sort of n <= C * THREADS * ITEMS keys; *done false:
 // this GPU cannot hold the cluster (nothing was launched).
-template <int ITEMS>
+template <int THREADS, int ITEMS>
 static cudaError_t launch_cluster(const uint64_t* keys, int32_t* vals, int64_t n, int passes, bool* done,
                                   cudaStream_t s) {
-    auto kern = k_sort_cluster<ITEMS>;
-    constexpr size_t smem = sizeof(CsShared<ITEMS>);
+    auto kern = k_sort_cluster<THREADS, ITEMS>;
+    constexpr size_t smem = sizeof(CsShared<THREADS, ITEMS>);
     static_assert(smem <= 232448, "227 KB of shared memory per CTA");
     int C = 1;
-    while ((int64_t)C * kCsThreads * ITEMS < n) C *= 2;
+    while ((int64_t)C * THREADS * ITEMS < n) C *= 2;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess && C > 8)
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)C);
-    cfg.blockDim = dim3(kCsThreads);
+    cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at{};
@@ -497,18 +535,18 @@ static cudaError_t launch_cluster(const uint64_t* keys, int32_t* vals, int64_t n
     return cudaLaunchKernelEx(&cfg, kern, keys, vals, (int)n, passes);
 }
 
-// As many CTAs as give each at least kCsThreads keys, up to the 16 of a
-// cluster, then more keys per thread.
+// As many CTAs as give each at least 512 keys, up to the 16 of a cluster, then
+// more threads, then more keys per thread.
 static cudaError_t launch_cluster_sort(const uint64_t* keys, int32_t* vals, int64_t n, int passes,
                                        bool* done, cudaStream_t s) {
     *done = false;
     if (n > kClusterSortMax) return cudaSuccess;
-    const int64_t per = (n + kCsMaxCluster * kCsThreads - 1) / (kCsMaxCluster * kCsThreads);
-    if (per <= 1) return launch_cluster<1>(keys, vals, n, passes, done, s);
-    if (per <= 2) return launch_cluster<2>(keys, vals, n, passes, done, s);
-    if (per <= 4) return launch_cluster<4>(keys, vals, n, passes, done, s);
-    if (per <= 8) return launch_cluster<8>(keys, vals, n, passes, done, s);
-    return launch_cluster<16>(keys, vals, n, passes, done, s);
+    const int64_t per = (n + kCsMaxCluster - 1) / kCsMaxCluster;  // keys per CTA of the largest cluster
+    if (per <= 512) return launch_cluster<512, 1>(keys, vals, n, passes, done, s);
+    if (per <= 1024) return launch_cluster<1024, 1>(keys, vals, n, passes, done, s);
+    if (per <= 2048) return launch_cluster<1024, 2>(keys, vals, n, passes, done, s);
+    if (per <= 4096) return launch_cluster<1024, 4>(keys, vals, n, passes, done, s);
+    return launch_cluster<1024, 8>(keys, vals, n, passes, done, s);
 }
 
 // Key buffer inside a sort scratch of sort_scratch_bytes(n) bytes.
