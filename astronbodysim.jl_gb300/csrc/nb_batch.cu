@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(kTileJ)
 // fills the GPU for 0.8 ms.  A part's sums go to global memory as compensated
 // pairs; the part that finishes last (a counter per split block) adds them in
 // part order, so the result does not depend on which CTA that is.  Integrating
-// that mix for 5 .. 15 steps took 56.5 ms unsplit and takes 21.8 ms.
+// that mix for 5 .. 15 steps took 56.5 ms unsplit and takes 19.4 ms.
 // ---------------------------------------------------------------------------
 // Launch shapes (threads per CTA, targets per thread); an item is one i-block
 // of BLOCK * IPT targets.  Default 128 x 2; the engine takes the shape from its
@@ -465,12 +465,15 @@ __device__ __forceinline__ void kick_particle(double* __restrict__ vx, double* _
     }
 }
 
-// Parts of a system's j-tiles: at least kPartTiles tiles each (the join then
-// costs below 1 % of a part), at most kMaxParts, and no more than it takes to
-// have kPartItems items, from where on the blocks alone balance the GPU.  A
-// rule on the system's own size, so a system is split the same way alone and
-// in any mix.
-constexpr int kPartTiles = 8, kMaxParts = 8, kPartItems = 4096;
+// Parts of a system's j-tiles: at least kPartTiles tiles each, at most
+// kMaxParts, and no more than it takes to have kPartItems items, from where on
+// the blocks alone balance the GPU.  A rule on the system's own size, so a
+// system is split the same way alone and in any mix.  GPU ms of 20 to 40 steps
+// with parts of 8 (at most 8), 4, 2 and 1 tiles (at most 16, 16, 32): 8 systems
+// of 500 to 6000 particles 6.3, 2.9, 1.6, 1.2; 160 of 64 to 8192 23.3, 22.6,
+// 22.4, 23.4; 12 of 413 to 45387 15.2, 14.7, 14.6, 14.5; 600 of 64 to 8192 29.5,
+// 29.5, 30.0, 31.6.
+constexpr int kPartTiles = 2, kMaxParts = 16, kPartItems = 4096;
 
 int batch_parts(int64_t n, int block, int ipt) {
     const int64_t nt = (n + kTileJ - 1) / kTileJ, bt = (int64_t)block * ipt, nb = (n + bt - 1) / bt;

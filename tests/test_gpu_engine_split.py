@@ -33,3 +33,31 @@ def test_split_systems_alone_and_in_the_mix(nb, law, shape):
         ref = nb.get_all_data(sim)
         np.testing.assert_allclose(got["pos"], ref["pos"], rtol=0, atol=1e-8)
         np.testing.assert_allclose(got["vel"], ref["vel"], rtol=0, atol=1e-6)
+
+
+@pytest.mark.parametrize("law", ["spline", "plummer"])
+def test_split_edges(nb, law):
+    """The first sizes that are split (4 tiles, the last of one source), the last
+    that are not, parts of 2 and 3 tiles, and the most parts with a partial last
+    tile: bit-identical alone and in a mix, and one step within the mixed form's
+    bar of the single-system path (each form's accelerations within 1e-4 of the
+    exact ones, so velocities within 2e-4 dt max|a| of each other)."""
+    sizes, dt, h = [255, 768, 769, 1500, 8100], 1e-3, 0.01
+    ds = [nb.plummer(n, seed=n) for n in sizes]
+    mix = nb.Engine(max_particles=1 << 16, max_systems=16, law=law)
+    ids = [mix.submit(d, h, dt, 1) for d in ds]
+    mix.run_until_idle()
+    for n, d, i in zip(sizes, ds, ids):
+        got = mix.fetch(i, n)
+        alone = nb.Engine(max_particles=1 << 16, max_systems=16, law=law)
+        k = alone.submit(d, h, dt, 1)
+        alone.run_until_idle()
+        a = alone.fetch(k, n)
+        np.testing.assert_array_equal(got["pos"], a["pos"])
+        np.testing.assert_array_equal(got["vel"], a["vel"])
+        sim = nb.Simulation(d, ForceSofteningTable=[h] * 6, TimeStep=dt, TimeEnd=1.0, law=law)
+        nb.run(sim, nsteps=1)
+        ref = nb.get_all_data(sim)
+        amax = np.abs(ref["acc"]).max()
+        assert np.abs(got["vel"] - ref["vel"]).max() <= 2e-4 * dt * amax
+        assert np.abs(got["pos"] - ref["pos"]).max() <= 2e-4 * dt * dt * amax
