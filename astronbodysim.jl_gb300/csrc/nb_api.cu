@@ -101,6 +101,11 @@ constexpr int kAutoJsplitMax = 8;
 // two, 11.9 by four, 11.1 by eight; N = 4096: 22.9, 21.6, 20.7, 20.4), and the
 // 15 steps between two sorts are not a multiple of eight.
 constexpr int64_t kManySteps = 4;
+// (block, part) items that a force over all particles aims at with blocks of 256
+// targets, from 65536 particles on: us a step with 6080 (nb::kSplitItems), 9120,
+// 12160, 18240 items at N = 65536 1464, 1462, 1463, 1470; N = 131072 5683, 5630,
+// 5607, 5592; N = 400001 51001, 50999, 50979, 50828.
+constexpr int64_t kWideItems = 12160;
 // Particles up to which nb_download joins evenly spaced arrays in one copy.
 constexpr int64_t kStridedCopyMax = 65536;
 constexpr ptrdiff_t kStridedCopyPitch = (ptrdiff_t)1 << 30;
@@ -430,8 +435,13 @@ cudaError_t enqueue_force(nb_handle* h, const nb::Targets& tg, cudaStream_t s, b
         js = h->auto_cfg ? nb::split_parts(nblk, h->ntiles) : 1;
         if (js * nblk * per > h->jslots) js = (int)(h->jslots / (nblk * per));
         if (nblk > h->ndone || js < 1) js = 1;
+    } else if (js == 0 && !active_only && per >= 256) {
+        js = (int)std::min<int64_t>(std::max<int64_t>(kWideItems / nblk, 8), (h->ntiles + 1) / 2);
+        if (js < 1) js = 1;
+    } else if (js > h->jalloc) {
+        js = 1;
     }
-    if (js == 0 || (js > 1 && (!particles || js <= h->jalloc))) {
+    if (js != 1) {
         src.jsplit = js;
         src.partial = h->jpartial;
         src.done = h->done;
@@ -615,9 +625,10 @@ int ensure_capacity(nb_handle* h, int64_t n) {
     // j-split partials: 8 floats per target slot and part (slots padded to 1024)
     const int64_t jstride = (n + 1023) / 1024 * 1024;
     int64_t jslots = js_need > 1 ? js_need * jstride : 0;
-    // the built-in split: at most kSplitItems rows of up to 256 targets where it exceeds 8 parts
+    // the built-in split: at most so many rows of its blocks' targets where it exceeds 8 parts
     if (h->auto_cfg) {
-        const int64_t few = std::min<int64_t>(nb::kSplitItems, jstride / 128 * ntiles) * 256;
+        const int64_t most = n >= kAutoIpt2From ? kWideItems * 256 : nb::kSplitItems * 128;
+        const int64_t few = std::min<int64_t>(most, jstride * ntiles);
         if (jslots < few) jslots = few;
     }
     size_t o_jp = take(sizeof(float) * 8 * (size_t)jslots);
