@@ -468,12 +468,14 @@ __device__ __forceinline__ void kick_particle(double* __restrict__ vx, double* _
 // Parts of a system's j-tiles: at least kPartTiles tiles each, at most
 // kMaxParts, and no more than it takes to have kPartItems items, from where on
 // the blocks alone balance the GPU.  A rule on the system's own size, so a
-// system is split the same way alone and in any mix.  GPU ms of 20 to 40 steps
-// with parts of 8 (at most 8), 4, 2 and 1 tiles (at most 16, 16, 32): 8 systems
-// of 500 to 6000 particles 6.3, 2.9, 1.6, 1.2; 160 of 64 to 8192 23.3, 22.6,
-// 22.4, 23.4; 12 of 413 to 45387 15.2, 14.7, 14.6, 14.5; 600 of 64 to 8192 29.5,
-// 29.5, 30.0, 31.6.
-constexpr int kPartTiles = 2, kMaxParts = 16, kPartItems = 4096;
+// system is split the same way alone and in any mix: few systems gain from
+// small parts, thousands pay for their joins.  GPU ms of 20 to 40 steps with
+// parts of 8 (at most 8), 4, 2 and 1 tiles (at most 16, 16, 32): 8 systems of
+// 500 to 6000 particles 6.3, 2.9, 1.6, 1.2; 160 of 64 to 8192 23.3, 22.6, 22.4,
+// 23.4; 12 of 413 to 45387 15.2, 14.7, 14.6, 14.5.  4096 systems of 64 to 8192:
+// 2525 G interactions/s unsplit, 2512, 2480 and 2407 with parts of 8, 4 and 2
+// tiles (2480 before the near loop's pass 2 was rewritten).
+constexpr int kPartTiles = 4, kMaxParts = 16, kPartItems = 4096;
 
 int batch_parts(int64_t n, int block, int ipt) {
     const int64_t nt = (n + kTileJ - 1) / kTileJ, bt = (int64_t)block * ipt, nb = (n + bt - 1) / bt;

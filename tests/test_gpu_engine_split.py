@@ -1,6 +1,6 @@
 """GPU test of the engine's force with the j-tiles of a system split over several
-work items: sizes at the edges of the rule (16 tiles of 256 are the fewest that
-are split), alone and in a mix (bit-identical), for every launch shape."""
+work items: sizes at and around the edges of the rule (8 tiles of 256 are the
+fewest that are split), alone and in a mix (bit-identical), for every launch shape."""
 import numpy as np
 import pytest
 
@@ -37,12 +37,12 @@ def test_split_systems_alone_and_in_the_mix(nb, law, shape):
 
 @pytest.mark.parametrize("law", ["spline", "plummer"])
 def test_split_edges(nb, law):
-    """The first sizes that are split (4 tiles, the last of one source), the last
-    that are not, parts of 2 and 3 tiles, and the most parts with a partial last
+    """The first sizes that are split (8 tiles, the last of one source), the last
+    that are not, parts of 4 and 6 tiles, and more parts with a partial last
     tile: bit-identical alone and in a mix, and one step within the mixed form's
     bar of the single-system path (each form's accelerations within 1e-4 of the
     exact ones, so velocities within 2e-4 dt max|a| of each other)."""
-    sizes, dt, h = [255, 768, 769, 1500, 8100], 1e-3, 0.01
+    sizes, dt, h = [255, 1792, 1793, 3000, 8100], 1e-3, 0.01
     ds = [nb.plummer(n, seed=n) for n in sizes]
     mix = nb.Engine(max_particles=1 << 16, max_systems=16, law=law)
     ids = [mix.submit(d, h, dt, 1) for d in ds]
