@@ -2,8 +2,7 @@
 //
 // Built with -fmad=false so every a*b+c rounds twice, as Julia evaluates the
 // pair expressions of src/directsum/gravity.jl:8-28 and
-// src/directsum/potential.jl:2-27; roots and quotients round as IEEE ones (see
-// root64 for the exceptions).  Each
+// src/directsum/potential.jl:2-27; sqrt and division are IEEE-rounded.  Each
 // pair term is therefore the same double the CPU computes; the per-target sum
 // is compensated (TwoSum), so the result differs from the CPU's pairwise sum
 // (src/directsum/gravity.jl:45) only by that sum's own rounding.
@@ -12,15 +11,19 @@
 // one target per thread.
 //
 // What bounds it: the FP64 pipe (2 lanes per clock and SM on this GPU), so the
-// time is FP64 operations / busy SMs.  A pair took about 60 with the compiler's
-// square root and division and TwoSum for the three sums; it takes 37 with G = 1 (40 otherwise) with one
-// reciprocal root for both (root64, quotient64) and sums ordered on the integer
-// pipe (ordered_sum_acc): 9.6 -> 13.4 G interactions/s on a full GPU, the same
-// terms to the last bit in every case measured.  One
+// time is FP64 operations / busy SMs.  Of a pair's operations 23 are its own:
+// the separation and its square (8), the products with it (3; 6 unless G = 1)
+// and the three sums, ordered on the integer pipe (ordered_sum_acc, 12 instead
+// of TwoSum's 21); the rest is one square root and one quotient, shared by force
+// and potential.  One
 // block of targets per CTA leaves most SMs idle below 152 x 8 blocks (N =
-// 4096: 32 CTAs on 152 SMs, 8.0 ms a force at the former rate), so each block's sources are
-// split over js CTAs (fp64_split) whose compensated partial sums are joined
-// in part order by k_force_fp64_join: 1.25 ms a step at N = 4096.
+// 4096: 32 CTAs on 152 SMs, 8.0 ms a force), so each block's sources are split
+// over js CTAs (fp64_split) whose compensated partial sums are joined in part
+// order by k_force_fp64_join: 1.31 ms a step at N = 4096, 12.5 G interactions/s
+// at N = 12000.
+// An own root and quotient from one reciprocal root took 1.24 ms there; their
+// terms were other doubles for subnormal masses (28 % of them at 2^-1060) and
+// the same elsewhere only as far as tried, so both are the compiler's.
 #include "nb_internal.cuh"
 
 namespace nb {
@@ -55,31 +58,6 @@ __device__ __forceinline__ void ordered_sum_acc(double& s, double& c, double v) 
     s = t;
 }
 
-// r = sqrt(x) and y ~ 1 / sqrt(x).  From the hardware's approximation y0 one
-// step of Halley's iteration, y = y0 (1 + e/2 + 3 e^2 / 8) with e = 1 - x y0^2,
-// then r = x y corrected by its residual (Markstein 1990), which rounds like
-// an exact square root but for cases within a 2^-50th of a tie.  8 FP64-pipe
-// operations and a square root's reciprocal for the quotients below, which
-// then need no division of their own.  x within 2^-300 .. 2^300 (in_range).
-__device__ __forceinline__ bool in_range(double x) {
-    return (uint32_t)(__double2hiint(x) - ((1023 - 300) << 20)) < (uint32_t)(600 << 20);
-}
-__device__ __forceinline__ void root64(double x, double& r, double& y) {
-    double y0;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(x));
-    const double e = __fma_rn(-__dmul_rn(x, y0), y0, 1.0);
-    y = __fma_rn(__dmul_rn(y0, e), __fma_rn(0.375, e, 0.5), y0);
-    const double g = __dmul_rn(x, y);
-    // y / 2 by its exponent
-    const double hy = __hiloint2double(__double2hiint(y) - (1 << 20), __double2loint(y));
-    r = __fma_rn(__fma_rn(-g, g, x), hy, g);
-}
-// m / d, z ~ 1 / d within a few ulp: the product corrected by its residual.
-__device__ __forceinline__ double quotient64(double m, double d, double z) {
-    const double q = __dmul_rn(m, z);
-    return __fma_rn(__fma_rn(-q, d, m), z, q);
-}
-
 // Pair at separation (dx, dy, dz): acceleration factor fac (times the
 // separation and G) and potential pot (with G).
 template <int LAW, bool ACC, bool POT>
@@ -87,23 +65,11 @@ __device__ __forceinline__ void pair64(double dx, double dy, double dz, double m
                                        double h_inv, double h3_inv, double& fac, double& pot) {
     const double r2 = dx * dx + dy * dy + dz * dz;
     const double x = LAW == NB_LAW_PLUMMER ? r2 + h * h : r2;
-    double r, y;
-    const bool fast = in_range(x);
-    if (fast) {
-        root64(x, r, y);
-    } else {
-        r = sqrt(x);
-        y = 0.0;
-    }
+    const double r = sqrt(x);
     // r >= h on the bit patterns: both are non-negative
     if (LAW == NB_LAW_PLUMMER || __double_as_longlong(r) >= __double_as_longlong(h)) {
-        if (fast) {
-            if (ACC) fac = quotient64(m, x * r, __dmul_rn(__dmul_rn(y, y), y));
-            if (POT) pot = -quotient64(m, r, y) * G;
-        } else {
-            if (ACC) fac = m / (x * r);
-            if (POT) pot = -m / r * G;
-        }
+        if (ACC) fac = m / (x * r);
+        if (POT) pot = -m / r * G;
         if (LAW == NB_LAW_PLUMMER && POT && r2 == 0.0) pot = pot * 0.0;
         return;
     }
