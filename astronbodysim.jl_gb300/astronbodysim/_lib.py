@@ -109,6 +109,7 @@ NB_REQ_RUNNING = 1
 NB_REQ_DONE = 2
 NB_REQ_CANCELLED = 3
 NB_REQ_SUSPENDED = 4
+NB_SELFTEST_FAIL_MOVE = 0
 NB_BG_NONE = 0
 NB_BG_POINT_MASS = 1
 NB_BG_PSEUDO_NEWTONIAN = 2
@@ -167,6 +168,7 @@ SIGNATURES = {
     "nb_batch_suspend": (ctypes.c_int, [_h, ctypes.c_int64]),
     "nb_batch_resume": (ctypes.c_int, [_h, ctypes.c_int64]),
     "nb_selftest_wait_timeout": (ctypes.c_int, [ctypes.c_int, ctypes.c_int64, _dp]),
+    "nb_selftest_engine": (ctypes.c_int, [_h, ctypes.c_int32, ctypes.c_int64]),
     "nb_selftest_fp32_peak": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, _dp, _dp]),
     "nb_checkpoint_size": (ctypes.c_int, [_h, _i64p]),
     "nb_checkpoint_save": (ctypes.c_int, [_h, _vp, ctypes.c_int64]),

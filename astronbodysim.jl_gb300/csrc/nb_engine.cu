@@ -107,6 +107,7 @@ struct nb_engine {
     void* stage = nullptr;   // device staging buffer, kStageBytes
     void* hstage = nullptr;  // its pinned host copy
     bool stage_failed = false;
+    int64_t fail_move = 0;   // self-test: the staged move that fails, counted from 1 (0: none)
     bool split = true;  // false: no memory for the partial sums, whole i-blocks instead
     uint32_t* derr = nullptr;
     int64_t tile_cap = 0;
@@ -485,21 +486,65 @@ double* stage_data(nb_engine* e) {
 }
 char* hstage_data(nb_engine* e) { return static_cast<char*>(e->hstage) + kStageTable; }
 
-int flush_admissions(nb_engine* e, MoveBatch& b) {
-    if (b.rows.empty()) return NB_OK;
+// The failure that nb_selftest_engine asked for, if this is its move.
+int planned_failure(nb_engine* e) {
+    if (e->fail_move > 0 && --e->fail_move == 0)
+        return efail(e, NB_ERR_CUDA, "staged move failed (self-test)");
+    return NB_OK;
+}
+
+// A system whose particles are in the arena runs.
+void mark_running(nb_engine* e, Request& q, int64_t off, int32_t slot, std::vector<int32_t>& admitted) {
+    q.in.clear();
+    q.in.shrink_to_fit();
+    q.order.clear();
+    q.order.shrink_to_fit();
+    q.aoff = off;
+    q.slot = slot;
+    q.state = NB_REQ_RUNNING;
+    if (!q.resumed) admitted.push_back(slot);  // a resumed system needs no start-up
+    q.resumed = false;
+    e->dirty = true;
+}
+
+// Gives the ranges and slots of the batch back; its systems head the queue again.
+void return_to_queue(nb_engine* e, MoveBatch& b) {
+    for (size_t k = b.rows.size(); k-- > 0;) {
+        free_range(e, b.rows[k].aoff, b.rows[k].n);
+        e->slot_req[b.rows[k].slot] = -1;
+        e->queue.push_front(b.reqs[k]->id);
+    }
+    b.clear();
+}
+
+int copy_admissions(nb_engine* e, const MoveBatch& b) {
+    int rc = planned_failure(e);
+    if (rc) return rc;
     std::memcpy(e->hstage, b.rows.data(), sizeof(nb::BatchMove) * b.rows.size());
     for (size_t k = 0; k < b.rows.size(); ++k) {
         Request& q = *b.reqs[k];
         std::memcpy(hstage_data(e) + sizeof(double) * (size_t)b.rows[k].src, q.in.data(),
                     sizeof(double) * 7 * (size_t)q.n);
-        q.in.clear();
-        q.in.shrink_to_fit();
     }
     NE_CK(cudaMemcpyAsync(e->stage, e->hstage, kStageTable + sizeof(double) * (size_t)b.doubles,
                           cudaMemcpyHostToDevice, e->stream));
     NE_CK(nb::launch_batch_admit(stage_table(e), (int32_t)b.rows.size(), b.max_n, stage_data(e),
                                  arena_arrays(e), e->stream));
     NE_CK(cudaStreamSynchronize(e->stream));  // before the staging buffer is filled again
+    return NB_OK;
+}
+
+// The batch's systems run once their particles are in the arena, not before: a
+// failed copy leaves them queued, with the particles that were submitted.
+int flush_admissions(nb_engine* e, MoveBatch& b, std::vector<int32_t>& admitted) {
+    if (b.rows.empty()) return NB_OK;
+    const int rc = copy_admissions(e, b);
+    if (rc) {
+        return_to_queue(e, b);
+        return rc;
+    }
+    for (size_t k = 0; k < b.rows.size(); ++k)
+        mark_running(e, *b.reqs[k], b.rows[k].aoff, b.rows[k].slot, admitted);
     b.clear();
     return NB_OK;
 }
@@ -527,10 +572,6 @@ int admit_alone(nb_engine* e, Request& q, int64_t off, int32_t slot) {
     }
     NE_CK(nb::launch_fill_i32(e->sysid + off, q.n, slot, e->stream));
     NE_CK(cudaStreamSynchronize(e->stream));
-    q.in.clear();
-    q.in.shrink_to_fit();
-    q.order.clear();
-    q.order.shrink_to_fit();
     return NB_OK;
 }
 
@@ -547,26 +588,28 @@ int admit(nb_engine* e, std::vector<int32_t>& admitted) {
         const int64_t off = alloc_range(e, q.n);
         if (off < 0) break;  // head of the queue waits for space (FIFO)
         const int64_t doubles = 7 * q.n;
-        if (!q.resumed && doubles <= kStageDoubles && have_stage(e)) {
-            if (!batch.fits(doubles)) {
-                int rc = flush_admissions(e, batch);
-                if (rc) return rc;
+        const bool staged = !q.resumed && doubles <= kStageDoubles && have_stage(e);
+        if (!staged || !batch.fits(doubles)) {
+            int rc = flush_admissions(e, batch, admitted);
+            if (rc) {
+                free_range(e, off, q.n);
+                return rc;
             }
+        }
+        if (staged) {
             batch.add(&q, off, slot, doubles);
         } else {
             int rc = admit_alone(e, q, off, slot);
-            if (rc) return rc;
+            if (rc) {
+                free_range(e, off, q.n);
+                return rc;
+            }
+            mark_running(e, q, off, slot, admitted);
         }
-        q.aoff = off;
-        q.slot = slot;
-        q.state = NB_REQ_RUNNING;
         e->slot_req[slot] = q.id;
         e->queue.pop_front();
-        if (!q.resumed) admitted.push_back(slot);  // a resumed system needs no start-up
-        q.resumed = false;
-        e->dirty = true;
     }
-    return flush_admissions(e, batch);
+    return flush_admissions(e, batch, admitted);
 }
 
 // Kick the given slots by fac (+0.5 on admission, -0.5 on retirement).
@@ -675,13 +718,14 @@ int prepare_chunk(nb_engine* e) {
     int rc = retire(e);  // systems submitted with nsteps == 0 or finished earlier
     if (rc) return rc;
     std::vector<int32_t> admitted;
-    rc = admit(e, admitted);
-    if (rc) return rc;
-    if (e->dirty) {
-        rc = rebuild(e);
-        if (rc) return rc;
-    }
-    return start_systems(e, admitted);
+    const int failed = admit(e, admitted);
+    const std::string why = failed ? e->err : std::string();
+    // the systems admitted before a failed copy are started all the same
+    if (e->dirty) rc = rebuild(e);
+    if (!rc) rc = start_systems(e, admitted);
+    if (!failed) return rc;
+    e->err = why;
+    return failed;
 }
 
 // Launch up to max_steps engine steps (at most max_steps_per_call, and no more
@@ -1072,6 +1116,14 @@ int nb_engine_drain_done(nb_engine* e, int64_t* ids, int64_t cap, int64_t* count
     e->finished.erase(e->finished.begin(), e->finished.begin() + k);
     *count = k;
     return NB_OK;
+}
+
+int nb_selftest_engine(nb_engine* e, int32_t what, int64_t value) {
+    if (!e || value < 0) return NB_ERR_INVALID_ARG;
+    switch (what) {
+        case NB_SELFTEST_FAIL_MOVE: e->fail_move = value; return NB_OK;
+        default: return efail(e, NB_ERR_INVALID_ARG, "unknown engine self-test %d", what);
+    }
 }
 
 const char* nb_engine_last_error(nb_engine* e) {

@@ -394,6 +394,14 @@ const char *nb_engine_last_error(nb_engine *e);
  * *waited_ms; the device context stays usable. */
 int nb_selftest_wait_timeout(int device, int64_t timeout_ns, double *waited_ms);
 
+/* Self-test of the engine's host paths (no counterpart in the reference), set
+ * on one engine:
+ *   NB_SELFTEST_FAIL_MOVE   the value-th batch of systems copied to or from the
+ *                           arena from now on fails with NB_ERR_CUDA before
+ *                           anything is copied (0: none). */
+#define NB_SELFTEST_FAIL_MOVE 0
+int nb_selftest_engine(nb_engine *e, int32_t what, int64_t value);
+
 /* FP32 throughput probe (no counterpart in the reference; it measures the
  * denominator of the force kernel's roofline): 4 CTAs x 256 threads per SM,
  * each thread running 8 independent chains of fma.rn.f32 (packed = 0) or
