@@ -60,6 +60,7 @@ struct Request {
     int32_t state = NB_REQ_QUEUED;
     int32_t slot = -1;
     int64_t aoff = -1;
+    bool kicked_back = false;  // the -1/2 kick of its retirement is made
     // suspended state: in = x, y, z, vx, vy, vz, m, ax, ay, az (n each), order = lperm
     bool resumed = false;
     std::vector<int32_t> order;
@@ -647,8 +648,22 @@ int start_systems(nb_engine* e, const std::vector<int32_t>& slots) {
     return half_kick(e, slots, 0.5);
 }
 
+// A system whose particles are back on the host is done.
+void mark_done(nb_engine* e, Request& q) {
+    free_range(e, q.aoff, q.n);
+    e->slot_req[q.slot] = -1;
+    q.state = NB_REQ_DONE;
+    e->stats.done += 1;
+    e->finished.push_back(q.id);
+    e->dirty = true;
+}
+
+// The batch's systems are done once their particles are on the host: after a
+// failed copy they wait in the arena for the next call.
 int flush_retirements(nb_engine* e, MoveBatch& b) {
     if (b.rows.empty()) return NB_OK;
+    const int rc = planned_failure(e);
+    if (rc) return rc;
     std::memcpy(e->hstage, b.rows.data(), sizeof(nb::BatchMove) * b.rows.size());
     NE_CK(cudaMemcpyAsync(e->stage, e->hstage, sizeof(nb::BatchMove) * b.rows.size(),
                           cudaMemcpyHostToDevice, e->stream));
@@ -661,55 +676,59 @@ int flush_retirements(nb_engine* e, MoveBatch& b) {
         Request& q = *b.reqs[k];
         std::memcpy(q.out.data(), hstage_data(e) + sizeof(double) * (size_t)b.rows[k].src,
                     sizeof(double) * 6 * (size_t)q.n);
+        mark_done(e, q);
     }
     b.clear();
     return NB_OK;
 }
 
+int retire_alone(nb_engine* e, Request& q) {
+    const size_t d = sizeof(double) * (size_t)q.n;
+    const double* src[6] = {e->x, e->y, e->z, e->vx, e->vy, e->vz};
+    for (int k = 0; k < 6; ++k)
+        NE_CK(cudaMemcpyAsync(q.out.data() + (size_t)k * q.n, src[k] + q.aoff, d,
+                              cudaMemcpyDeviceToHost, e->stream));
+    NE_CK(nb::launch_fill_i32(e->sysid + q.aoff, q.n, -1, e->stream));
+    NE_CK(cudaStreamSynchronize(e->stream));
+    mark_done(e, q);
+    return NB_OK;
+}
+
 // Retire systems whose step count is reached: -1/2 kick, download, free.
 int retire(nb_engine* e) {
-    std::vector<int32_t> fin;
+    std::vector<int32_t> fin, kick;
     for (int32_t s = 0; s < (int32_t)e->slot_req.size(); ++s) {
         if (e->slot_req[s] < 0) continue;
         Request& q = e->reqs[e->slot_req[s]];
-        if (q.state == NB_REQ_RUNNING && q.steps_done >= q.nsteps) fin.push_back(s);
+        if (q.state != NB_REQ_RUNNING || q.steps_done < q.nsteps) continue;
+        fin.push_back(s);
+        if (!q.kicked_back) kick.push_back(s);
     }
     if (fin.empty()) return NB_OK;
-    int rc = half_kick(e, fin, -0.5);
-    if (rc) return rc;
+    int rc = NB_OK;
+    if (!kick.empty()) {
+        rc = half_kick(e, kick, -0.5);
+        if (rc) return rc;
+        for (int32_t s : kick) e->reqs[e->slot_req[s]].kicked_back = true;
+    }
     MoveBatch batch;
     for (int32_t s : fin) {
         Request& q = e->reqs[e->slot_req[s]];
         q.out.resize((size_t)6 * q.n);
         const int64_t doubles = 6 * q.n;
-        if (doubles <= kStageDoubles && have_stage(e)) {
-            if (!batch.fits(doubles)) {
-                rc = flush_retirements(e, batch);
-                if (rc) return rc;
-            }
-            batch.add(&q, q.aoff, s, doubles);
-            continue;
+        const bool staged = doubles <= kStageDoubles && have_stage(e);
+        if (!staged || !batch.fits(doubles)) {
+            rc = flush_retirements(e, batch);
+            if (rc) return rc;
         }
-        const size_t d = sizeof(double) * (size_t)q.n;
-        const double* src[6] = {e->x, e->y, e->z, e->vx, e->vy, e->vz};
-        for (int k = 0; k < 6; ++k)
-            NE_CK(cudaMemcpyAsync(q.out.data() + (size_t)k * q.n, src[k] + q.aoff, d,
-                                  cudaMemcpyDeviceToHost, e->stream));
-        NE_CK(nb::launch_fill_i32(e->sysid + q.aoff, q.n, -1, e->stream));
-        NE_CK(cudaStreamSynchronize(e->stream));
+        if (staged) {
+            batch.add(&q, q.aoff, s, doubles);
+        } else {
+            rc = retire_alone(e, q);
+            if (rc) return rc;
+        }
     }
-    rc = flush_retirements(e, batch);
-    if (rc) return rc;
-    for (int32_t s : fin) {
-        Request& q = e->reqs[e->slot_req[s]];
-        free_range(e, q.aoff, q.n);
-        q.state = NB_REQ_DONE;
-        e->slot_req[s] = -1;
-        e->stats.done += 1;
-        e->finished.push_back(q.id);
-        e->dirty = true;
-    }
-    return NB_OK;
+    return flush_retirements(e, batch);
 }
 
 // Admission and start-up before a chunk of steps: retire finished systems,

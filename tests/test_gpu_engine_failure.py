@@ -60,3 +60,22 @@ def test_selftest_arguments(nb):
     assert f(eng.handle, 99, 1) == L.NB_ERR_INVALID_ARG
     assert f(eng.handle, L.NB_SELFTEST_FAIL_MOVE, -1) == L.NB_ERR_INVALID_ARG
     assert f(None, L.NB_SELFTEST_FAIL_MOVE, 1) == L.NB_ERR_INVALID_ARG
+
+
+@pytest.mark.parametrize("which,done", [(1, 0), (2, 8)])
+def test_failed_retirement(nb, undisturbed, which, done):
+    """20000 particles take 0.96 MB on the way back, eight to a batch.  Those
+    copied before the failure are done; the others are kicked back once."""
+    L = nb._lib
+    eng = _engine(nb)
+    ids = _submit(nb, eng)
+    assert eng.run(1) == 1
+    assert L.load().nb_selftest_engine(eng.handle, L.NB_SELFTEST_FAIL_MOVE, which) == L.NB_OK
+    with pytest.raises(L.NbodyError) as err:
+        eng.run(1)
+    assert err.value.code == L.NB_ERR_CUDA
+    states = [eng.poll(i)[0] for i in ids]
+    assert states == [L.NB_REQ_DONE] * done + [L.NB_REQ_RUNNING] * (len(ids) - done)
+    assert eng.drain_done() == ids[:done]
+    _finish(eng, ids, undisturbed)
+    assert eng.drain_done() == ids[done:]
