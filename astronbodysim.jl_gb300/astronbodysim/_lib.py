@@ -110,6 +110,7 @@ NB_REQ_DONE = 2
 NB_REQ_CANCELLED = 3
 NB_REQ_SUSPENDED = 4
 NB_SELFTEST_FAIL_MOVE = 0
+NB_SELFTEST_PARTIAL_ROWS = 1
 NB_BG_NONE = 0
 NB_BG_POINT_MASS = 1
 NB_BG_PSEUDO_NEWTONIAN = 2

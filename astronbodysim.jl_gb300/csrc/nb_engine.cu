@@ -48,6 +48,18 @@ constexpr size_t kStageTable = sizeof(nb::BatchMove) * kStageMoves;
 constexpr size_t kStageBytes = (size_t)8 << 20;
 constexpr int64_t kStageDoubles = (int64_t)((kStageBytes - kStageTable) / sizeof(double));
 
+// Most memory for the partial sums of split systems.  A step whose sums take
+// more runs its work items in several launches, each within the buffer; at 1 GiB
+// a launch has 14 ms of work or more, against some 50 us that its end costs.
+constexpr size_t kPartialBytes = (size_t)1 << 30;
+
+// Work items [first, first + count) that run in one launch of the batch force.
+struct ItemGroup {
+    int64_t first = 0;
+    int32_t count = 0;
+    int32_t nsplit = 0;  // split blocks among them
+};
+
 struct Request {
     int64_t id = 0;
     int64_t n = 0;
@@ -101,15 +113,17 @@ struct nb_engine {
     nb::BatchItem* items = nullptr;
     nb::BatchItem* items_new = nullptr;
     int32_t* counter = nullptr;
-    // partial sums of the systems whose j-tiles are split: grown in rebuild()
-    // to what the running systems need, freed with the engine
+    // rows of partial sums for the systems whose j-tiles are split: at first one
+    // block's, in the arena; grown in rebuild() up to kPartialBytes while there is
+    // memory, freed with the engine
     float* partial = nullptr;
-    size_t partial_floats = 0;
+    int64_t rows = 0;
+    void* grown = nullptr;   // the allocation behind partial, if it has grown
+    int64_t row_limit = 0;   // self-test: most rows (0: no limit)
     void* stage = nullptr;   // device staging buffer, kStageBytes
     void* hstage = nullptr;  // its pinned host copy
     bool stage_failed = false;
     int64_t fail_move = 0;   // self-test: the staged move that fails, counted from 1 (0: none)
-    bool split = true;  // false: no memory for the partial sums, whole i-blocks instead
     uint32_t* derr = nullptr;
     int64_t tile_cap = 0;
     int64_t item_cap = 0;
@@ -124,8 +138,7 @@ struct nb_engine {
     bool dirty = true;
     int32_t nrank = 0;
     int32_t ntiles_total = 0;
-    int32_t nitems = 0;
-    int32_t nsplit = 0;  // split blocks among them
+    std::vector<ItemGroup> groups;  // the work items of a step, by launch
     int32_t max_small_n = 0;   // largest system ordered in shared memory
     // systems too large for the shared-memory sort ("large"): their ranks,
     // particle count and largest size; they are radix-sorted every step
@@ -221,20 +234,56 @@ int check_err(nb_engine* e) {
     return NB_OK;
 }
 
-// Appends the work items of the system of rank r: its i-blocks, each in
-// batch_parts() parts.  prow and nsplit count the rows of partial sums and the
-// split blocks so far.
-void add_items(nb_engine* e, std::vector<nb::BatchItem>& items, int32_t r, const nb::SysDesc& d,
-               int64_t& prow, int32_t& nsplit) {
-    const int32_t parts = e->split ? nb::batch_parts(d.n, e->fblock, e->fipt) : 1;
-    for (int32_t b = 0; b < d.nblocks; ++b) {
-        for (int32_t k = 0; k < parts; ++k)
-            items.push_back(nb::BatchItem{r, b, k, parts, (int32_t)prow, nsplit});
-        if (parts > 1) {
-            prow += parts;
-            nsplit += 1;
+// Work items of systems: their i-blocks, each in batch_parts() parts, in
+// launches whose partial sums fit in `rows` rows (at least one block's).  How a
+// system is split depends on its size alone, so its results depend neither on
+// the memory that the sums get nor on the other systems.
+struct ItemList {
+    std::vector<nb::BatchItem> items;
+    std::vector<ItemGroup> groups;
+    int64_t rows = 0;
+    int64_t prow = 0;  // rows of the last launch
+
+    void add(nb_engine* e, int32_t r, const nb::SysDesc& d) {
+        const int32_t parts = nb::batch_parts(d.n, e->fblock, e->fipt);
+        for (int32_t b = 0; b < d.nblocks; ++b) {
+            if (groups.empty() || (parts > 1 && prow + parts > rows)) {
+                groups.push_back(ItemGroup{(int64_t)items.size(), 0, 0});
+                prow = 0;
+            }
+            ItemGroup& g = groups.back();
+            for (int32_t k = 0; k < parts; ++k)
+                items.push_back(nb::BatchItem{r, b, k, parts, (int32_t)prow, g.nsplit});
+            g.count += parts;
+            if (parts > 1) {
+                prow += parts;
+                g.nsplit += 1;
+            }
         }
     }
+};
+
+// Makes room for up to `need` rows of partial sums, as far as kPartialBytes and
+// the memory go; the old buffer serves until there is a larger one.  Grows by
+// half at least, so a mix that grows does not allocate each time.
+void grow_partial(nb_engine* e, int64_t need) {
+    const size_t row = sizeof(float) * nb::batch_partial_row(e->fblock, e->fipt);
+    int64_t most = (int64_t)(kPartialBytes / row);
+    if (e->row_limit > 0) most = std::min(most, e->row_limit);
+    if (need <= e->rows || e->rows >= most) return;
+    int64_t want = std::min(most, std::max(need, e->rows + e->rows / 2));
+    void* p = nullptr;
+    while (want > e->rows && cudaMalloc(&p, row * (size_t)want) != cudaSuccess) {
+        (void)cudaGetLastError();
+        p = nullptr;
+        want /= 2;
+    }
+    if (!p) return;
+    drop_graph(e);  // it holds the old buffer's address
+    if (e->grown) cudaFree(e->grown);
+    e->grown = p;
+    e->partial = static_cast<float*>(p);
+    e->rows = want;
 }
 
 // Rebuild the rank tables of the running systems and upload them.
@@ -287,31 +336,16 @@ int rebuild(nb_engine* e) {
     for (int32_t r = 0; r < R; ++r) order[r] = r;
     std::stable_sort(order.begin(), order.end(),
                      [&](int32_t a, int32_t b) { return sd[a].ntiles > sd[b].ntiles; });
-    std::vector<nb::BatchItem> items;
-    int64_t prow = 0;
-    int32_t nsplit = 0;
-    e->split = true;
-    for (int32_t r : order) add_items(e, items, r, sd[r], prow, nsplit);
-    const size_t pf = (size_t)prow * nb::batch_partial_row(e->fblock, e->fipt);
-    if (pf > e->partial_floats) {
-        if (e->partial) cudaFree(e->partial);
-        e->partial = nullptr;
-        e->partial_floats = 0;
-        const cudaError_t me = cudaMalloc(&e->partial, sizeof(float) * pf);
-        if (me == cudaSuccess) {
-            e->partial_floats = pf;
-        } else if (me == cudaErrorMemoryAllocation) {
-            (void)cudaGetLastError();
-            e->partial = nullptr;
-            e->split = false;
-            items.clear();
-            prow = 0;
-            nsplit = 0;
-            for (int32_t r : order) add_items(e, items, r, sd[r], prow, nsplit);
-        } else {
-            NE_CK(me);
-        }
+    int64_t need = 0;
+    for (const nb::SysDesc& d : sd) {
+        const int32_t parts = nb::batch_parts(d.n, e->fblock, e->fipt);
+        if (parts > 1) need += (int64_t)parts * d.nblocks;
     }
+    grow_partial(e, need);
+    ItemList list;
+    list.rows = e->rows;
+    for (int32_t r : order) list.add(e, r, sd[r]);
+    const std::vector<nb::BatchItem>& items = list.items;
     if (toff > e->tile_cap) return efail(e, NB_ERR_STATE, "tile capacity exceeded");
     if ((int64_t)items.size() > e->item_cap) return efail(e, NB_ERR_STATE, "work-item capacity exceeded");
     if (R > 0) {
@@ -326,8 +360,7 @@ int rebuild(nb_engine* e) {
     NE_CK(cudaMemcpy(e->nsteps_slot, nst.data(), sizeof(int64_t) * nst.size(), cudaMemcpyHostToDevice));
     e->nrank = R;
     e->ntiles_total = (int32_t)toff;
-    e->nitems = (int32_t)items.size();
-    e->nsplit = nsplit;
+    e->groups = std::move(list.groups);
     e->high_water = hw;
     e->max_small_n = 0;
     for (int32_t r = 0; r < R; ++r)
@@ -343,12 +376,12 @@ int rebuild(nb_engine* e) {
     return NB_OK;
 }
 
-nb::BatchForce force_args(nb_engine* e, const nb::BatchItem* items, int32_t nitems, int32_t nsplit) {
+nb::BatchForce force_args(nb_engine* e, const nb::BatchItem* items, const ItemGroup& g) {
     nb::BatchForce f{};
     f.sys = e->sysdesc;
-    f.items = items;
-    f.nitems = nitems;
-    f.nsplit = nsplit;
+    f.items = items + g.first;
+    f.nitems = g.count;
+    f.nsplit = g.nsplit;
     f.counter = e->counter;
     f.partial = e->partial;
     f.perm = e->lperm;
@@ -421,17 +454,19 @@ cudaError_t enqueue_step(nb_engine* e, cudaStream_t s, bool gated) {
     // force with the step's kick fused into its epilogue: every target of the
     // work items is a particle of a running system, and those are exactly
     // the particles the kick moves (fac_step 1)
-    nb::BatchForce f = force_args(e, e->items, e->nitems, e->nsplit);
-    f.vx = e->vx;
-    f.vy = e->vy;
-    f.vz = e->vz;
-    f.sysid = e->sysid;
-    f.dt_slot = e->dt_slot;
-    f.fac_slot = e->fac_step;
-    f.steps_slot = e->steps_slot;
-    f.nsteps_slot = nsteps;
-    r = nb::launch_force_batch(e->p.law, f, e->occ_acc * e->nsm, e->fblock, e->fipt, s);
-    if (r != cudaSuccess) return r;
+    for (const ItemGroup& g : e->groups) {
+        nb::BatchForce f = force_args(e, e->items, g);
+        f.vx = e->vx;
+        f.vy = e->vy;
+        f.vz = e->vz;
+        f.sysid = e->sysid;
+        f.dt_slot = e->dt_slot;
+        f.fac_slot = e->fac_step;
+        f.steps_slot = e->steps_slot;
+        f.nsteps_slot = nsteps;
+        r = nb::launch_force_batch(e->p.law, f, e->occ_acc * e->nsm, e->fblock, e->fipt, s);
+        if (r != cudaSuccess) return r;
+    }
     return nb::launch_batch_tick(e->batchsys, e->nrank, e->steps_slot, nsteps, s);
 }
 
@@ -634,17 +669,17 @@ int start_systems(nb_engine* e, const std::vector<int32_t>& slots) {
     for (int32_t s : slots) ranks.push_back(ros[s]);
     std::stable_sort(ranks.begin(), ranks.end(),
                      [&](int32_t a, int32_t b) { return sd[a].ntiles > sd[b].ntiles; });
-    std::vector<nb::BatchItem> items;
-    int64_t prow = 0;
-    int32_t nsplit = 0;
-    for (int32_t r : ranks) add_items(e, items, r, sd[r], prow, nsplit);
-    NE_CK(cudaMemcpy(e->items_new, items.data(), sizeof(nb::BatchItem) * items.size(),
+    ItemList list;
+    list.rows = e->rows;
+    for (int32_t r : ranks) list.add(e, r, sd[r]);
+    NE_CK(cudaMemcpy(e->items_new, list.items.data(), sizeof(nb::BatchItem) * list.items.size(),
                      cudaMemcpyHostToDevice));
     // New systems have step count 0, so they are due for ordering; the others
     // keep their order (their schedule must not depend on admissions).
     NE_CK(enqueue_sort_pack(e, e->stream, false, false));
-    NE_CK(nb::launch_force_batch(e->p.law, force_args(e, e->items_new, (int32_t)items.size(), nsplit),
-                                 e->occ_acc * e->nsm, e->fblock, e->fipt, e->stream));
+    for (const ItemGroup& g : list.groups)
+        NE_CK(nb::launch_force_batch(e->p.law, force_args(e, e->items_new, g), e->occ_acc * e->nsm,
+                                     e->fblock, e->fipt, e->stream));
     return half_kick(e, slots, 0.5);
 }
 
@@ -877,6 +912,8 @@ int nb_engine_create(const nb_engine_params* p, nb_engine** out) {
     e->item_cap = blocks * nb::batch_max_parts();
     size_t o_it = take(sizeof(nb::BatchItem) * (size_t)e->item_cap);
     size_t o_itn = take(sizeof(nb::BatchItem) * (size_t)e->item_cap);
+    const int64_t rows = nb::batch_max_parts();  // one block's partial sums
+    size_t o_par = take(sizeof(float) * nb::batch_partial_row(e->fblock, e->fipt) * (size_t)rows);
     size_t o_cnt = take(sizeof(int32_t) * (size_t)(1 + blocks)), o_err = take(sizeof(uint32_t) * 4);
     if (cudaMalloc(&e->arena, off) != cudaSuccess) {
         cudaStreamDestroy(e->stream);
@@ -907,6 +944,8 @@ int nb_engine_create(const nb_engine_params* p, nb_engine** out) {
     e->box_key = (unsigned long long*)(b + o_bk);
     e->items = (nb::BatchItem*)(b + o_it);
     e->items_new = (nb::BatchItem*)(b + o_itn);
+    e->partial = (float*)(b + o_par);
+    e->rows = rows;
     e->counter = (int32_t*)(b + o_cnt);
     e->derr = (uint32_t*)(b + o_err);
     cudaMemset(e->derr, 0, sizeof(uint32_t));
@@ -934,7 +973,7 @@ int nb_engine_destroy(nb_engine* e) {
     drop_graph(e);
     if (e->ev0) cudaEventDestroy(e->ev0);
     if (e->ev1) cudaEventDestroy(e->ev1);
-    if (e->partial) cudaFree(e->partial);
+    if (e->grown) cudaFree(e->grown);
     if (e->stage) cudaFree(e->stage);
     if (e->hstage) cudaFreeHost(e->hstage);
     cudaFree(e->arena);
@@ -1141,6 +1180,7 @@ int nb_selftest_engine(nb_engine* e, int32_t what, int64_t value) {
     if (!e || value < 0) return NB_ERR_INVALID_ARG;
     switch (what) {
         case NB_SELFTEST_FAIL_MOVE: e->fail_move = value; return NB_OK;
+        case NB_SELFTEST_PARTIAL_ROWS: e->row_limit = value; return NB_OK;
         default: return efail(e, NB_ERR_INVALID_ARG, "unknown engine self-test %d", what);
     }
 }

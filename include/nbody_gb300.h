@@ -398,8 +398,11 @@ int nb_selftest_wait_timeout(int device, int64_t timeout_ns, double *waited_ms);
  * on one engine:
  *   NB_SELFTEST_FAIL_MOVE   the value-th batch of systems copied to or from the
  *                           arena from now on fails with NB_ERR_CUDA before
- *                           anything is copied (0: none). */
+ *                           anything is copied (0: none);
+ *   NB_SELFTEST_PARTIAL_ROWS  the buffer of partial sums grows to value rows at
+ *                           most, as if memory ended there (0: no limit). */
 #define NB_SELFTEST_FAIL_MOVE 0
+#define NB_SELFTEST_PARTIAL_ROWS 1
 int nb_selftest_engine(nb_engine *e, int32_t what, int64_t value);
 
 /* FP32 throughput probe (no counterpart in the reference; it measures the
