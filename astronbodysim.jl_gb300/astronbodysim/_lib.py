@@ -130,6 +130,7 @@ class nb_diag(ctypes.Structure):
 _dp = ctypes.POINTER(ctypes.c_double)
 _i32p = ctypes.POINTER(ctypes.c_int32)
 _i64p = ctypes.POINTER(ctypes.c_int64)
+_u64p = ctypes.POINTER(ctypes.c_uint64)
 _vp = ctypes.c_void_p
 _h = ctypes.c_void_p
 
@@ -169,6 +170,8 @@ SIGNATURES = {
     "nb_batch_suspend": (ctypes.c_int, [_h, ctypes.c_int64]),
     "nb_batch_resume": (ctypes.c_int, [_h, ctypes.c_int64]),
     "nb_selftest_wait_timeout": (ctypes.c_int, [ctypes.c_int, ctypes.c_int64, _dp]),
+    "nb_selftest_copy_runs": (ctypes.c_int, [ctypes.c_int32, _u64p, _u64p, ctypes.c_int64, ctypes.c_int32,
+                                             _u64p, _u64p, _i32p]),
     "nb_selftest_engine": (ctypes.c_int, [_h, ctypes.c_int32, ctypes.c_int64]),
     "nb_selftest_fp32_peak": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, _dp, _dp]),
     "nb_checkpoint_size": (ctypes.c_int, [_h, _i64p]),

@@ -11,6 +11,9 @@
 #include <string>
 #include <vector>
 
+#include <cuda.h>
+
+#include "nb_copy_runs.h"
 #include "nb_internal.cuh"
 
 using nb::Clock;
@@ -108,7 +111,7 @@ constexpr int64_t kManySteps = 4;
 constexpr int64_t kWideItems = 12160;
 // Particles up to which nb_download joins evenly spaced arrays in one copy.
 constexpr int64_t kStridedCopyMax = 65536;
-constexpr ptrdiff_t kStridedCopyPitch = (ptrdiff_t)1 << 30;
+constexpr size_t kStridedCopyPitch = (size_t)1 << 30;
 constexpr int64_t kAutoTile256From = 1 << 15;
 constexpr int64_t kAutoIpt2From = 1 << 16;
 constexpr int64_t kAutoTile512From = 1 << 17;
@@ -937,9 +940,32 @@ int nb_upload(nb_handle* h, int64_t n, const double* x, const double* y, const d
     return upload_sysdesc(h);
 }
 
-static bool pinned_host(const void* p) {
-    cudaPointerAttributes a{};
-    return cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type == cudaMemoryTypeHost;
+// The pinned host allocation that holds p (empty: none, or not known).
+static nb::HostRange pinned_range(uintptr_t p) {
+    using Query = CUresult(CUDAAPI*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Query query = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q{};
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 7000, cudaEnableDefault, &q) !=
+                cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            (void)cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<Query>(f);
+    }();
+    nb::HostRange r;
+    if (!query) return r;
+    unsigned type = 0, managed = 0;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    CUpointer_attribute attr[4] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                   CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* data[4] = {&type, &managed, &start, &size};
+    if (query(4, attr, data, (CUdeviceptr)p) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST || managed) return r;
+    r.lo = (uintptr_t)start;
+    r.hi = r.lo + size;
+    return r;
 }
 
 int nb_download(nb_handle* h, double* x, double* y, double* z, double* vx, double* vy, double* vz,
@@ -954,25 +980,21 @@ int nb_download(nb_handle* h, double* x, double* y, double* z, double* vx, doubl
     double* const dst[10] = {x, y, z, vx, vy, vz, ax, ay, az, pot};
     const double* const src[10] = {h->x,  h->y,  h->z,  h->vx, h->vy, h->vz,
                                    h->ax, h->ay, h->az, h->pot};
-    // The arena's arrays are evenly spaced.  Runs of pinned host arrays that are
-    // so too go as one strided copy while the copies' own cost counts (ten steps
-    // of N = 1000 with the download of nine arrays: 221 -> 202 us).
-    const ptrdiff_t pitch = (const char*)h->y - (const char*)h->x;
+    // The arena's arrays are evenly spaced.  Runs of rows of one pinned host
+    // allocation that are so too go as one strided copy while the copies' own
+    // cost counts (ten steps of N = 1000 with the download of nine arrays: 221 ->
+    // 202 us).
+    uintptr_t da[10], sa[10];
+    for (int k = 0; k < 10; ++k) {
+        da[k] = (uintptr_t)dst[k];
+        sa[k] = (uintptr_t)src[k];
+    }
     for (int k = 0; k < 10;) {
-        int rows = 1;
-        if (dst[k] && h->n <= kStridedCopyMax) {
-            const ptrdiff_t step = k + 1 < 10 && dst[k + 1] ? (char*)dst[k + 1] - (char*)dst[k] : 0;
-            while (step >= (ptrdiff_t)d && step <= kStridedCopyPitch && k + rows < 10 && dst[k + rows] &&
-                   (char*)dst[k + rows] - (char*)dst[k + rows - 1] == step &&
-                   (const char*)src[k + rows] - (const char*)src[k + rows - 1] == pitch)
-                ++rows;
-            if (rows > 1 &&
-                !(pinned_host(dst[k]) && pinned_host(dst[k + rows - 1]) &&
-                  cudaMemcpy2DAsync(dst[k], (size_t)step, src[k], (size_t)pitch, d, (size_t)rows,
-                                    cudaMemcpyDeviceToHost, s) == cudaSuccess)) {
-                (void)cudaGetLastError();
-                rows = 1;
-            }
+        int rows = h->n <= kStridedCopyMax ? nb::copy_run(da, sa, 10, k, d, kStridedCopyPitch, pinned_range) : 1;
+        if (rows > 1 && cudaMemcpy2DAsync(dst[k], da[k + 1] - da[k], src[k], sa[k + 1] - sa[k], d, (size_t)rows,
+                                          cudaMemcpyDeviceToHost, s) != cudaSuccess) {
+            (void)cudaGetLastError();
+            rows = 1;
         }
         if (dst[k] && rows == 1) NB_CK(cudaMemcpyAsync(dst[k], src[k], d, cudaMemcpyDeviceToHost, s));
         k += rows;
@@ -1595,6 +1617,30 @@ int nb_checkpoint_load(nb_handle* h, const void* buf, int64_t bytes) {
     h->perm_valid = order_ok;
     h->host_steps = order_ok ? hd.order_steps : 0;
     return upload_sysdesc(h);
+}
+
+int nb_selftest_copy_runs(int32_t rows, const uint64_t* dst, const uint64_t* src, int64_t bytes,
+                          int32_t ranges, const uint64_t* lo, const uint64_t* hi, int32_t* run) {
+    if (rows < 1 || rows > 64 || !dst || !src || bytes < 1 || ranges < 0 || (ranges > 0 && (!lo || !hi)) || !run)
+        return NB_ERR_INVALID_ARG;
+    uintptr_t d[64], s[64];
+    for (int k = 0; k < rows; ++k) {
+        d[k] = (uintptr_t)dst[k];
+        s[k] = (uintptr_t)src[k];
+        run[k] = 0;
+    }
+    auto range_of = [&](uintptr_t p) {
+        nb::HostRange r;
+        for (int j = 0; j < ranges; ++j)
+            if (p >= lo[j] && p < hi[j]) {
+                r.lo = (uintptr_t)lo[j];
+                r.hi = (uintptr_t)hi[j];
+            }
+        return r;
+    };
+    for (int k = 0; k < rows; k += run[k])
+        run[k] = nb::copy_run(d, s, rows, k, (size_t)bytes, kStridedCopyPitch, range_of);
+    return NB_OK;
 }
 
 const char* nb_last_error(nb_handle* h) {

@@ -405,6 +405,14 @@ int nb_selftest_wait_timeout(int device, int64_t timeout_ns, double *waited_ms);
 #define NB_SELFTEST_PARTIAL_ROWS 1
 int nb_selftest_engine(nb_engine *e, int32_t what, int64_t value);
 
+/* Self-test of the download's choice of strided copies, on the host (no
+ * counterpart in the reference): rows of `bytes` bytes at dst[k] (0: not
+ * wanted) from src[k], with the pinned host allocations [lo[j], hi[j]).
+ * run[k] = rows that one copy writes from row k on (1 also for a row not wanted;
+ * 0: within an earlier run). */
+int nb_selftest_copy_runs(int32_t rows, const uint64_t *dst, const uint64_t *src, int64_t bytes,
+                          int32_t ranges, const uint64_t *lo, const uint64_t *hi, int32_t *run);
+
 /* FP32 throughput probe (no counterpart in the reference; it measures the
  * denominator of the force kernel's roofline): 4 CTAs x 256 threads per SM,
  * each thread running 8 independent chains of fma.rn.f32 (packed = 0) or
