@@ -172,6 +172,8 @@ SIGNATURES = {
     "nb_selftest_wait_timeout": (ctypes.c_int, [ctypes.c_int, ctypes.c_int64, _dp]),
     "nb_selftest_copy_runs": (ctypes.c_int, [ctypes.c_int32, _u64p, _u64p, ctypes.c_int64, ctypes.c_int32,
                                              _u64p, _u64p, _i32p]),
+    "nb_selftest_cluster_join": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,
+                                                _dp, _dp, _dp]),
     "nb_selftest_engine": (ctypes.c_int, [_h, ctypes.c_int32, ctypes.c_int64]),
     "nb_selftest_fp32_peak": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, _dp, _dp]),
     "nb_checkpoint_size": (ctypes.c_int, [_h, _i64p]),

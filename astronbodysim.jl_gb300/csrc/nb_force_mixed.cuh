@@ -263,8 +263,13 @@ __device__ __forceinline__ void end_constant_step(const Targets& tg) {
 // the sums' round trip through the L2, the count, and most of the time of the
 // FP64 epilogue, which one CTA's threads otherwise share the FP64 pipe of one
 // SM for: 5.7 of 19.5 us of a force launch at N = 4096, 3.7 of 7.4 at N = 1000.
+// A part whose wait ran out (gave_up, CTA-uniform) leaves a mark in place of its
+// sums, a NaN that no sum can be, and then no CTA of the block stores, kicks or
+// advances the clock.
+constexpr uint32_t kGaveUp = 0x7fe0dead;
+
 template <int BLOCK, int IPT>
-__device__ __forceinline__ void cluster_join(float* sum, int js, int part, int64_t base, int64_t ntg,
+__device__ __forceinline__ void cluster_join(float* sum, bool gave_up, int js, int part, int64_t base, int64_t ntg,
                                              const float* sx, const float* cx, const float* sy,
                                              const float* cy, const float* sz, const float* cz,
                                              const Targets& tg, double G) {
@@ -283,7 +288,12 @@ __device__ __forceinline__ void cluster_join(float* sum, int js, int part, int64
         q[4 * kPer] = sz[k];
         q[5 * kPer] = cz[k];
     }
+    if (gave_up)
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+            for (int k = 0; k < IPT; ++k) sum[2 * j * kPer + k * BLOCK + tid] = __uint_as_float(kGaveUp);
     const int seg = (kPer + js - 1) / js, lo = part * seg;
+    bool whole = true;
     cluster.sync();
     for (int i = tid; i < 3 * seg; i += BLOCK) {
         const int comp = i / seg, slot = lo + i % seg;
@@ -297,14 +307,18 @@ __device__ __forceinline__ void cluster_join(float* sum, int js, int part, int64
 #pragma unroll 8
         for (int u = 0; u < js; ++u) {
             const float* q = cluster.map_shared_rank(sum + 2 * comp * kPer + slot, u);
-            two_sum_acc(s, c, q[0]);
+            const float v = q[0];
+            whole = whole && __float_as_uint(v) != kGaveUp;
+            two_sum_acc(s, c, v);
             c += q[kPer];
         }
+        if (!whole) break;
         const double acc = ((double)s + (double)c) * G;
         a[p] = acc;
         if (v) v[p] = __dadd_rn(vp, __dmul_rn(acc, tg.kick_dt));  // k_kick with constant steps
     }
-    if (tg.step_clk && base == 0 && part == 0 && tid == 0) end_constant_step(tg);
+    // (this thread has joined the block's first target)
+    if (tg.step_clk && base == 0 && part == 0 && tid == 0 && whole) end_constant_step(tg);
     cluster.sync();  // the last read of another CTA's shared memory
 }
 
@@ -476,7 +490,7 @@ __global__ void __launch_bounds__(BLOCK, (ForceOcc<BLOCK, IPT, ACC, POT>::value)
 
     if constexpr (kClusterJoin<BLOCK, IPT, TJ, ACC, POT>) {
         if (src.cluster) {
-            cluster_join<BLOCK, IPT>(reinterpret_cast<float*>(buf), js, part, base, ntg, sx, cx, sy, cy, sz,
+            cluster_join<BLOCK, IPT>(reinterpret_cast<float*>(buf), abort_flag != 0u, js, part, base, ntg, sx, cx, sy, cy, sz,
                                      cz, tg, G);
             return;
         }

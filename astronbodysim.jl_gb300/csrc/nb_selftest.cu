@@ -5,7 +5,7 @@
 // the context stays usable.
 #include <cstdio>
 
-#include "nb_internal.cuh"
+#include "nb_force_mixed.cuh"
 
 namespace {
 
@@ -134,5 +134,64 @@ extern "C" int nb_selftest_fp32_peak(int device, int packed, double* tflops, dou
     if (e != cudaSuccess) return NB_ERR_CUDA;
     if (ms) *ms = best;
     if (tflops) *tflops = flop / (best * 1e-3) / 1e12;
+    return NB_OK;
+}
+
+// ---------------------------------------------------------------------------
+// Join of a block of 128 targets whose parts are one cluster, with sums that
+// the host can add up, and one part that gives up (gave_up; none: -1).
+// ---------------------------------------------------------------------------
+namespace {
+
+__global__ void __launch_bounds__(128) k_join_cluster(nb::Targets tg, int js, int gave_up) {
+    __shared__ float sum[6 * 128];
+    const int part = (int)blockIdx.x, t = (int)threadIdx.x;
+    // (sum, carry) of this part per component: 2^part + t and (component + 1) 2^-40
+    const float s[1] = {exp2f((float)part) + (float)t};
+    const float c0[1] = {exp2f(-40.0f)}, c1[1] = {2.0f * c0[0]}, c2[1] = {3.0f * c0[0]};
+    nb::cluster_join<128, 1>(sum, part == gave_up, js, part, 0, tg.n, s, c0, s, c1, s, c2, tg, 1.0);
+}
+
+}  // namespace
+
+extern "C" int nb_selftest_cluster_join(int device, int parts, int gave_up, int n, double* acc, double* vel,
+                                        double* t_float) {
+    if (parts < 1 || parts > nb::kClusterParts || gave_up >= parts || n < 1 || n > 128 || !acc || !vel || !t_float)
+        return NB_ERR_INVALID_ARG;
+    if (cudaSetDevice(device) != cudaSuccess) return NB_ERR_CUDA;
+    const size_t rows = sizeof(double) * 6 * 128;  // ax, ay, az, vx, vy, vz
+    char* mem = nullptr;
+    if (cudaMalloc(&mem, rows + sizeof(nb::Clock)) != cudaSuccess) return NB_ERR_OOM;
+    double* row = reinterpret_cast<double*>(mem);
+    nb::Targets tg{};
+    tg.n = n;
+    tg.ax = row;
+    tg.ay = row + 128;
+    tg.az = row + 2 * 128;
+    tg.vx = row + 3 * 128;
+    tg.vy = row + 4 * 128;
+    tg.vz = row + 5 * 128;
+    tg.kick_dt = 0.5;
+    tg.step_clk = reinterpret_cast<nb::Clock*>(mem + rows);
+    cudaMemset(mem, 0, rows + sizeof(nb::Clock));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)parts);
+    cfg.blockDim = dim3(128);
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)parts;
+    at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, k_join_cluster, tg, parts, gave_up);
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    nb::Clock c{};
+    if (e == cudaSuccess) e = cudaMemcpy(acc, row, rows / 2, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(vel, row + 3 * 128, rows / 2, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(&c, tg.step_clk, sizeof c, cudaMemcpyDeviceToHost);
+    cudaFree(mem);
+    if (e != cudaSuccess) return NB_ERR_CUDA;
+    *t_float = c.t_float;
     return NB_OK;
 }

@@ -394,6 +394,15 @@ const char *nb_engine_last_error(nb_engine *e);
  * *waited_ms; the device context stays usable. */
 int nb_selftest_wait_timeout(int device, int64_t timeout_ns, double *waited_ms);
 
+/* Self-test of the join of a block of n <= 128 targets whose `parts` <= 8 parts
+ * are one thread-block cluster (no counterpart in the reference).  Part u holds,
+ * for target t and component k, the sum 2^u + t with the carry (k + 1) 2^-40;
+ * part gave_up (-1: none) ends as one whose wait ran out.  acc, vel: 3 x 128
+ * values each, zero before, vel kicked by half of acc; *t_float: the clock,
+ * advanced by a half.  With a part that gave up all stay zero. */
+int nb_selftest_cluster_join(int device, int parts, int gave_up, int n, double *acc, double *vel,
+                             double *t_float);
+
 /* Self-test of the engine's host paths (no counterpart in the reference), set
  * on one engine:
  *   NB_SELFTEST_FAIL_MOVE   the value-th batch of systems copied to or from the
