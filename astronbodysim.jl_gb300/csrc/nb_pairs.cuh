@@ -30,14 +30,21 @@ struct LoopShape {
 };
 constexpr uint64_t kWaitTimeoutNs = 2000000000ull;  // 2 s
 
+// A separation other than zero, also where its square is none in FP32 (below
+// about 2e-23).
+__device__ __forceinline__ bool apart(float dx, float dy, float dz) {
+    return ((__float_as_uint(dx) | __float_as_uint(dy) | __float_as_uint(dz)) & 0x7fffffffu) != 0u;
+}
+
 // ---------------------------------------------------------------------------
 // Spline slow path (0 <= r < h), FP32, with hinv = 1/h and hinv3 = hinv^3.
 // Returns m*fac (to multiply d) in mr3 and the negated potential contribution
-// in mp.
+// in mp (none without a separation: a target's own entry).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void spline_close(float r2, float rinv, float m, float hinv, float hinv3,
+__device__ __forceinline__ void spline_close(float r2, float rinv, bool sep, float m, float hinv, float hinv3,
                                              float& mr3, float& mp) {
-    const float r = (r2 > 0.0f) ? r2 * rinv : 0.0f;
+    // rinv is infinite for subnormal r2
+    const float r = r2 >= 1.17549435e-38f ? r2 * rinv : __fsqrt_rn(r2);
     const float u = r * hinv;
     float fac, wp;
     if (u < 0.5f) {
@@ -51,7 +58,7 @@ __device__ __forceinline__ void spline_close(float r2, float rinv, float m, floa
              u * u * (10.666666666667f + u * (-16.0f + u * (9.6f - 2.133333333333f * u)));
     }
     mr3 = m * hinv3 * fac;
-    mp = (r2 > 0.0f) ? -(m * hinv * wp) : 0.0f;  // +m/r convention: phi contribution is -mp
+    mp = sep ? -(m * hinv * wp) : 0.0f;  // +m/r convention: phi contribution is -mp
 }
 
 // ---------------------------------------------------------------------------
@@ -388,8 +395,8 @@ __device__ __forceinline__ void pair_loop_checked_impl(const float4* __restrict_
     // any lane flagged, pair by pair with a vote each, was a serial chain of
     // some 130 cycles per pair: most of a small system's force time, since every
     // target's own entry flags a block.)
-    // A pair with r = 0, every target's own entry among them, needs no
-    // correction of the force: both terms are d times a finite factor, d = 0.
+    // A pair with d = 0, every target's own entry among them, needs no
+    // correction of the force: both terms are d times a finite factor.
     // Only its potential term goes.
 #pragma unroll
     for (int k = 0; k < IPT; ++k) {
@@ -406,8 +413,8 @@ __device__ __forceinline__ void pair_loop_checked_impl(const float4* __restrict_
                 const float2 dy = __fadd2_rn(make_float2(A.z, A.w), ny[k]);
                 const float2 dz = __fadd2_rn(make_float2(B.x, B.y), nz[k]);
                 const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-                hit |= (uint32_t)(r2.x < h2[k] && (POT || r2.x > 0.0f)) << (2 * i);
-                hit |= (uint32_t)(r2.y < h2[k] && (POT || r2.y > 0.0f)) << (2 * i + 1);
+                hit |= (uint32_t)(r2.x < h2[k] && (POT || apart(dx.x, dy.x, dz.x))) << (2 * i);
+                hit |= (uint32_t)(r2.y < h2[k] && (POT || apart(dx.y, dy.y, dz.y))) << (2 * i + 1);
             }
             for (; hit != 0u; hit &= hit - 1u) {
                 const int i = __ffs(hit) - 1, half = i & 1;
@@ -416,19 +423,20 @@ __device__ __forceinline__ void pair_loop_checked_impl(const float4* __restrict_
                 const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
                 const float mass = UNI ? mu : f[6];
                 float mr3, mp;
-                spline_close(r2, rsqrt_approx(r2), mass, hinv, hinv3, mr3, mp);
+                const bool sep = apart(dx, dy, dz);
+                spline_close(r2, rsqrt_approx(r2), sep, mass, hinv, hinv3, mr3, mp);
                 // minus the clamped Newtonian term of pass 1, m r_h^-3 d and m r_h^-1
                 const float mrh = mass * rh;
                 const float d3 = mr3 - (mrh * rh) * rh;
                 if (half == 0) {
-                    if (r2 > 0.0f) {
+                    if (sep) {
                         tx[k].x = fmaf(dx, d3, tx[k].x);
                         ty[k].x = fmaf(dy, d3, ty[k].x);
                         tz[k].x = fmaf(dz, d3, tz[k].x);
                     }
                     if (POT) tp[k].x += mp - mrh;
                 } else {
-                    if (r2 > 0.0f) {
+                    if (sep) {
                         tx[k].y = fmaf(dx, d3, tx[k].y);
                         ty[k].y = fmaf(dy, d3, ty[k].y);
                         tz[k].y = fmaf(dz, d3, tz[k].y);
