@@ -1594,6 +1594,7 @@ int nb_checkpoint_load(nb_handle* h, const void* buf, int64_t bytes) {
     }
     h->n = n;
     h->ntiles = (int32_t)((n + h->tj - 1) / h->tj);
+    hd.clk.ticket = 0;  // no part of the state: images may hold any word here
     NB_CK(cudaMemcpy(h->clk, &hd.clk, sizeof(Clock), cudaMemcpyHostToDevice));
     if (n == 0) return NB_OK;
     size_t off = sizeof hd;
