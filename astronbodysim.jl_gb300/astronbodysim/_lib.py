@@ -111,6 +111,7 @@ NB_REQ_CANCELLED = 3
 NB_REQ_SUSPENDED = 4
 NB_SELFTEST_FAIL_MOVE = 0
 NB_SELFTEST_PARTIAL_ROWS = 1
+NB_SELFTEST_NO_STAGING = 2
 NB_BG_NONE = 0
 NB_BG_POINT_MASS = 1
 NB_BG_PSEUDO_NEWTONIAN = 2
@@ -174,6 +175,8 @@ SIGNATURES = {
                                              _u64p, _u64p, _i32p]),
     "nb_selftest_cluster_join": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                                 _dp, _dp, _dp]),
+    "nb_selftest_sort": (ctypes.c_int, [ctypes.c_int, ctypes.c_int64, _u64p, ctypes.c_int, ctypes.c_int,
+                                        _i32p]),
     "nb_selftest_engine": (ctypes.c_int, [_h, ctypes.c_int32, ctypes.c_int64]),
     "nb_selftest_fp32_peak": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, _dp, _dp]),
     "nb_checkpoint_size": (ctypes.c_int, [_h, _i64p]),

@@ -1181,6 +1181,10 @@ int nb_selftest_engine(nb_engine* e, int32_t what, int64_t value) {
     switch (what) {
         case NB_SELFTEST_FAIL_MOVE: e->fail_move = value; return NB_OK;
         case NB_SELFTEST_PARTIAL_ROWS: e->row_limit = value; return NB_OK;
+        case NB_SELFTEST_NO_STAGING:
+            if (e->stage) return efail(e, NB_ERR_STATE, "the staging buffers are there already");
+            e->stage_failed = value != 0;
+            return NB_OK;
         default: return efail(e, NB_ERR_INVALID_ARG, "unknown engine self-test %d", what);
     }
 }

@@ -385,7 +385,8 @@ size_t sort_scratch_bytes(int64_t n);
 cudaError_t launch_morton_sort(const double* x, const double* y, const double* z, int64_t n,
                                void* scratch, int32_t* perm, cudaStream_t s);
 uint64_t* sort_keys_buffer(void* scratch, int64_t n);
-cudaError_t launch_sort_keys(void* scratch, int64_t n, int32_t* vals, int passes, cudaStream_t s);
+cudaError_t launch_sort_keys(void* scratch, int64_t n, int32_t* vals, int passes, cudaStream_t s,
+                             bool chain = false);
 // Tile sizes of the packed sources: 128, 256 or 512 (src.tile_j); stages:
 // depth of the force kernel's shared-memory ring (3, 4, 6; see
 // nb_force_mixed.cuh for the combinations compiled).

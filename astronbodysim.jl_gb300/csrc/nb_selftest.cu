@@ -195,3 +195,22 @@ extern "C" int nb_selftest_cluster_join(int device, int parts, int gave_up, int 
     *t_float = c.t_float;
     return NB_OK;
 }
+
+extern "C" int nb_selftest_sort(int device, int64_t n, const uint64_t* keys, int passes, int chain, int32_t* perm) {
+    if (n < 1 || n > (int64_t)1 << 24 || !keys || !perm || passes < 2 || passes > 8 || passes % 2)
+        return NB_ERR_INVALID_ARG;
+    if (cudaSetDevice(device) != cudaSuccess) return NB_ERR_CUDA;
+    const size_t scratch = nb::sort_scratch_bytes(n);  // a multiple of 256
+    char* mem = nullptr;
+    if (cudaMalloc(&mem, scratch + sizeof(int32_t) * (size_t)n) != cudaSuccess) return NB_ERR_OOM;
+    int32_t* vals = reinterpret_cast<int32_t*>(mem + scratch);
+    for (int64_t i = 0; i < n; ++i) perm[i] = (int32_t)i;
+    cudaError_t e = cudaMemcpy(vals, perm, sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess)
+        e = cudaMemcpy(nb::sort_keys_buffer(mem, n), keys, sizeof(uint64_t) * (size_t)n, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = nb::launch_sort_keys(mem, n, vals, passes, nullptr, chain != 0);
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e == cudaSuccess) e = cudaMemcpy(perm, vals, sizeof(int32_t) * (size_t)n, cudaMemcpyDeviceToHost);
+    cudaFree(mem);
+    return e == cudaSuccess ? NB_OK : NB_ERR_CUDA;
+}

@@ -553,12 +553,13 @@ static cudaError_t launch_cluster_sort(const uint64_t* keys, int32_t* vals, int6
 uint64_t* sort_keys_buffer(void* scratch, int64_t n) { return carve(scratch, n).keys_a; }
 
 // Stable LSD radix sort of (keys, vals): keys in sort_keys_buffer(scratch, n),
-// vals (n int32) in place; `passes` 8-bit digits from the bottom (even).
-cudaError_t launch_sort_keys(void* scratch, int64_t n, int32_t* vals, int passes, cudaStream_t s) {
+// vals (n int32) in place; `passes` 8-bit digits from the bottom (even).  chain:
+// without the cluster sort.
+cudaError_t launch_sort_keys(void* scratch, int64_t n, int32_t* vals, int passes, cudaStream_t s, bool chain) {
     if (n <= 0) return cudaSuccess;
     SortScratch sc = carve(scratch, n);
     bool done = false;
-    cudaError_t e = launch_cluster_sort(sc.keys_a, vals, n, passes, &done, s);
+    cudaError_t e = chain ? cudaSuccess : launch_cluster_sort(sc.keys_a, vals, n, passes, &done, s);
     if (e != cudaSuccess || done) return e;
     const int nblocks = (int)sort_blocks(n);
     uint64_t* kin = sc.keys_a;

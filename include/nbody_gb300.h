@@ -403,15 +403,23 @@ int nb_selftest_wait_timeout(int device, int64_t timeout_ns, double *waited_ms);
 int nb_selftest_cluster_join(int device, int parts, int gave_up, int n, double *acc, double *vel,
                              double *t_float);
 
+/* Self-test of the radix sort (no counterpart in the reference): perm = the
+ * stable order of n keys by their lowest `passes` bytes (2, 4, 6 or 8).  chain 1:
+ * by the chain of kernels, as on a GPU without room for the cluster. */
+int nb_selftest_sort(int device, int64_t n, const uint64_t *keys, int passes, int chain, int32_t *perm);
+
 /* Self-test of the engine's host paths (no counterpart in the reference), set
  * on one engine:
  *   NB_SELFTEST_FAIL_MOVE   the value-th batch of systems copied to or from the
  *                           arena from now on fails with NB_ERR_CUDA before
  *                           anything is copied (0: none);
  *   NB_SELFTEST_PARTIAL_ROWS  the buffer of partial sums grows to value rows at
- *                           most, as if memory ended there (0: no limit). */
+ *                           most, as if memory ended there (0: no limit);
+ *   NB_SELFTEST_NO_STAGING  value 1: as if there were no memory for the staging
+ *                           buffers (before the first system moves). */
 #define NB_SELFTEST_FAIL_MOVE 0
 #define NB_SELFTEST_PARTIAL_ROWS 1
+#define NB_SELFTEST_NO_STAGING 2
 int nb_selftest_engine(nb_engine *e, int32_t what, int64_t value);
 
 /* Self-test of the download's choice of strided copies, on the host (no
