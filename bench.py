@@ -37,11 +37,14 @@ EPS = 1.0e-3
 DT = 1.0e-4
 FLOP_PER_INTERACTION = 20
 L2_FLUSH_BYTES = 256 << 20
-# kernels in one step graph at N = 2^20: clock advance, drift, 2 bounding-box,
-# Morton keys, 8 radix passes x (histogram, 3-kernel scan, scatter), pack,
-# force, kick, clock end; plus the join of a j-split force (or the fix-up of
-# the work-list force)
-STEP_KERNELS = 49
+
+
+def step_kernels(n, worklist=False):
+    """Kernels in one constant step with its sort: drift, bounding box, Morton
+    keys, the sort (one cluster kernel up to 131072 particles, else 8 passes of
+    histogram, 3-kernel scan, scatter), pack, force with join, kick and clock; the
+    work-list force has a fix-up, clock advance, kick and clock end of their own."""
+    return 5 + (1 if n <= 1 << 17 else 40) + (4 if worklist else 0)
 
 
 def dist_env():
@@ -550,7 +553,7 @@ def run_gpu(args):
                                          "built-in rule of the library"),)))},
             "roofline": {"bound": "fp32", "achieved": achieved, "peak": fp32_peak_tflops,
                          "unit": "TFLOP/s", "frac": achieved / fp32_peak_tflops, "traffic": traffic,
-                         "kernel": "k_force_mixed (+k_pack, k_force_join)", "force_ms": force_ms,
+                         "kernel": "k_force_mixed (+k_pack)", "force_ms": force_ms,
                          "peak_note": ("of measured: fma.rn.f32x2 throughput of this GPU (nb_selftest_fp32_peak); "
                                        "nominal SMs x 128 lanes x 2 x %.0f MHz = %.1f TFLOP/s; 20 flop/interaction"
                                        % (sm_max, nominal_tflops)) if fp32_measured else
@@ -561,7 +564,7 @@ def run_gpu(args):
             "cpu_baseline": cpu,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h, "steps": args.e2e_steps},
-            "gpu_launches": (STEP_KERNELS + (1 if tuned_eff[2] > 1 or tuned_eff[0] == -1 else 0)) * args.steps,
+            "gpu_launches": step_kernels(n, tuned_eff[0] == -1) * args.steps,
             "clocks": clocks,
             "accuracy": acc_stats,
             "general_mass": extra.get("general_mass"),
