@@ -299,8 +299,8 @@ bool fused_step(const nb_handle* h) {
 }
 
 // An adaptive step by the kernels of launch_adaptive_start: mixed precision on
-// the direct grid, with nothing between the force and the kick.  Five kernels
-// beside the force instead of ten.
+// the direct grid, with nothing between the force and the kick.  Four kernels
+// beside the force (start, pack, list, kick) instead of eleven.
 bool lean_adaptive_step(const nb_handle* h) {
     return h->p.precision == NB_PREC_MIXED && h->p.adaptive && !h->worklist &&
            h->p.bg_kind == NB_BG_NONE && h->p.mond == NB_MOND_NONE;

@@ -471,10 +471,10 @@ __device__ __forceinline__ void kick_particle(double* __restrict__ vx, double* _
 // system is split the same way alone and in any mix: few systems gain from
 // small parts, thousands pay for their joins.  GPU ms of 20 to 40 steps with
 // parts of 8 (at most 8), 4, 2 and 1 tiles (at most 16, 16, 32): 8 systems of
-// 500 to 6000 particles 6.3, 2.9, 1.6, 1.2; 160 of 64 to 8192 23.3, 22.6, 22.4,
-// 23.4; 12 of 413 to 45387 15.2, 14.7, 14.6, 14.5.  4096 systems of 64 to 8192:
-// 2525 G interactions/s unsplit, 2512, 2480 and 2407 with parts of 8, 4 and 2
-// tiles (2480 before the near loop's pass 2 was rewritten).
+// 500 to 6000 particles 6.3, 2.9, 1.6, 1.2; 160 of 64 to 8192 23.4, 22.7, 22.5,
+// 23.4 (unsplit 27.1); 12 of 413 to 45387 15.3, 14.7, 14.6, 14.6 (unsplit 47.8).
+// 4096 systems of 64 to 8192: 2565 G interactions/s unsplit, 2550, 2516, 2432 and
+// 2245 with parts of 8, 4, 2 and 1 tiles; 600 such: 2433, 2461, 2450, 2388, 2216.
 constexpr int kPartTiles = 4, kMaxParts = 16, kPartItems = 4096;
 
 int batch_parts(int64_t n, int block, int ipt) {

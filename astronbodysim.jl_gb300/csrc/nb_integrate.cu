@@ -317,11 +317,12 @@ cudaError_t launch_sync_count(const int64_t* ti_end, int64_t n, const Clock* clk
 }
 
 // ---------------------------------------------------------------------------
-// The adaptive step in five kernels beside the pack and the force's own: start
-// (min end step, clock), [pack: drift, counts], list, [force], kick (with the
-// clock's end of the step).  It took eleven (three for the start, three for the
-// list, drift, kick and clock of their own), of which a substep with few active
-// particles is mostly made: 12 substeps of 2 x 16384 particles 1205 -> 1096 us.
+// The adaptive step in three kernels beside the pack and the force: start
+// (min end step, clock), [pack: drift, counts], list (behind a scan above 131072
+// particles), [force], kick (with the clock's end of the step).  It took nine (two
+// for the end step, three for the list, drift, kick and two clock kernels of their
+// own), of which a substep with few active particles is mostly made: 12 substeps
+// of 2 x 16384 particles 1205 -> 1096 us.
 // ---------------------------------------------------------------------------
 constexpr int64_t kStartBlocks = 1216;
 
